@@ -97,26 +97,32 @@ Engine::Engine(const Config &config) : params(config) {
     }
     tables_.root_reduced = upload_table(rc);
     tables_.root_inverse_reduced = upload_table(ric);
-    // Plain twiddles and their Shoup quotients for shoup_mult.
-    std::vector<int64_t> rs(2 * rc.size()), ris(2 * ric.size());
+    // Plain twiddles with their Shoup quotients (shoup_mult), or as doubles beside the
+    // scaled Montgomery words (fp_prime).
+    std::vector<int64_t> rs(2 * static_cast<size_t>(P) * p.n), ris(rs.size());
     for (int i = 0; i < P; i++) {
-      const uint64_t qi = p.q[i];
-      using u128 = unsigned __int128;
-      auto mulmod = [&](uint64_t a, uint64_t b) { return static_cast<uint64_t>(static_cast<u128>(a) * b % qi); };
-      uint64_t r_inverse = 1, base = (uint64_t(1) << 62) % qi;  // R^-1 = R^(q-2) mod q
-      for (uint64_t e = qi - 2; e > 0; e >>= 1) {
-        if (e & 1) r_inverse = mulmod(r_inverse, base);
-        base = mulmod(base, base);
-      }
-      auto pair = [&](int64_t mont, int64_t *out) {
-        const uint64_t w = mulmod(static_cast<uint64_t>(mont), r_inverse);
-        out[0] = static_cast<int64_t>(w);
-        out[1] = static_cast<int64_t>((static_cast<u128>(w) << 64) / qi);
+      const uint64_t qi = p.q[i], ki = p.k[i];
+      auto plain = [&](int64_t mont) {  // times R^-1
+        return static_cast<uint64_t>(guard(mont_exit(mont, qi, ki), static_cast<int64_t>(qi)));
       };
-      for (size_t j = 0; j < per; j++) {
-        pair(rc[i * per + j], &rs[2 * (i * per + j)]);
-        pair(ric[i * per + j], &ris[2 * (i * per + j)]);
-      }
+      if (fp_prime(qi)) tables_.fp_primes.add(i);
+      auto fill = [&](const std::vector<int64_t> &mont, const std::vector<int64_t> &reduced,
+                      std::vector<int64_t> &out, int shift) {
+        int64_t *o = &out[2 * static_cast<size_t>(i) * p.n];
+        const int64_t *in = &reduced[i * per], *word = &mont[i * per];
+        for (size_t j = 0; j < per; j++) {
+          const uint64_t w = plain(in[j]);
+          if (fp_prime(qi)) {
+            o[j + shift] = static_cast<int64_t>(fp_raw(static_cast<double>(w)));
+            o[p.n + j + shift] = static_cast<int64_t>(fp_raw(static_cast<double>(word[j]) * kFpMontScale));
+          } else {
+            o[2 * j] = static_cast<int64_t>(w);
+            o[2 * j + 1] = static_cast<int64_t>((static_cast<unsigned __int128>(w) << 64) / qi);
+          }
+        }
+      };
+      fill(p.root, rc, rs, 1);
+      fill(p.root_inverse, ric, ris, 0);
     }
     tables_.root_shoup = upload_table(rs);
     tables_.root_inverse_shoup = upload_table(ris);
@@ -196,7 +202,7 @@ Engine::Engine(const Config &config) : params(config) {
       }
     }
     ks_.rescale_enter_shoup = upload_table(resh);
-    ks_.r_mod = upload_table(rmod);
+    tables_.r_mod = upload_table(rmod);
     // P mod q and its Shoup quotient (the tensor addend of the key inner product):
     // p_product_mult_r R^-1.
     std::vector<int64_t> psh(2 * static_cast<size_t>(P), 0);

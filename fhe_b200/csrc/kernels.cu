@@ -20,9 +20,10 @@ NttTuning g_ntt_tuning[18];  // zero: the default
 
 NttTuning ntt_default_tuning(int log_n) {
   NttTuning t;
-  t.s_second = log_n >= 15 ? 8 : (log_n >= 13 ? 7 : 6);
-  t.first_columns_log = log_n - t.s_second >= 9 ? 3 : 4;
-  t.second_tile_log = 12;
+  // Tiles of 2048 words, what ntt_pass_fp works on.
+  t.s_second = log_n >= 13 ? log_n - ntt_strided_stages(log_n) : 6;
+  t.first_columns_log = kNttFpTileLog - (log_n - t.s_second);
+  t.second_tile_log = kNttFpTileLog;
   return t;
 }
 
@@ -494,72 +495,6 @@ __global__ void __launch_bounds__(256)
   mod_down_store(t, ks, n, moduli_id, L, poly, coeff0, valid, ops, out, first_limb, divide);
 }
 
-struct TensorLoad {
-  const int64_t *a;
-  const int64_t *b;
-  long long poly_stride;  // limbs * n
-  const uint64_t *q;
-  const uint64_t *k;
-  // Optional sink of the third polynomial's NTT-form words into each partition's own
-  // limbs of ModUp's extended buffer [count][extended][N].
-  int64_t *own_ext = nullptr;
-  const int *part_start = nullptr;
-  const int *part_size = nullptr;
-  int part_count = 0;
-  int extended = 0;
-  bool third_only = false;  // a one-polynomial launch of the third polynomial
-  __device__ __forceinline__ int64_t operator()(int poly, int limb, int prime, int gi, int n) const {
-    const long long i = static_cast<long long>(limb) * n + gi;
-    const uint64_t qq = q[prime], kk = k[prime];
-    if (third_only) poly = 2;
-    if (poly == 0) return mont_mult_lazy(a[i], b[i], qq, kk);
-    if (poly == 2) {
-      const int64_t v = mont_mult_lazy(a[poly_stride + i], b[poly_stride + i], qq, kk);
-      if (own_ext != nullptr) {
-        int p = 0;
-        while (p + 1 < part_count && limb >= part_start[p] + part_size[p]) p++;
-        own_ext[(static_cast<long long>(p) * extended + limb) * n + gi] = v;
-      }
-      return v;
-    }
-    const int64_t qs = static_cast<int64_t>(qq);
-    return guard(guard(mont_mult_lazy(a[i], b[poly_stride + i], qq, kk) +
-                           mont_mult_lazy(a[poly_stride + i], b[i], qq, kk),
-                       qs << 1),
-                 qs);
-  }
-};
-
-// The tensor's third polynomial d2 = a1 b1 as a streaming pass before a plain mixed
-// inverse transform (TensorLoad's words, with 16-byte accesses by a full grid: the
-// loader pass of d2 alone waits on its loads and fills under one wave), and its
-// NTT-form words into each partition's own limbs of ModUp's extended buffer when one
-// is given.  Same words either way.
-__global__ void __launch_bounds__(256)
-    tensor_third_kernel(PrimeTables t, TensorLoad ld, int log_n, int limbs, int prime_base,
-                        int64_t *y) {
-  const long long pairs = static_cast<long long>(limbs) << (log_n - 1);
-  const long long n = 1LL << log_n;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < pairs;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long w = 2 * i;
-    const int limb = static_cast<int>(w >> log_n);
-    const int prime = prime_base + limb;
-    const uint64_t q = t.q[prime], k = t.k[prime];
-    const longlong2 a = *reinterpret_cast<const longlong2 *>(ld.a + ld.poly_stride + w);
-    const longlong2 b = *reinterpret_cast<const longlong2 *>(ld.b + ld.poly_stride + w);
-    longlong2 v;
-    v.x = mont_mult_lazy(a.x, b.x, q, k);
-    v.y = mont_mult_lazy(a.y, b.y, q, k);
-    *reinterpret_cast<longlong2 *>(y + w) = v;
-    if (ld.own_ext != nullptr) {
-      int p = 0;
-      while (p + 1 < ld.part_count && limb >= ld.part_start[p] + ld.part_size[p]) p++;
-      *reinterpret_cast<longlong2 *>(ld.own_ext + (static_cast<long long>(p) * ld.extended) * n + w) = v;
-    }
-  }
-}
-
 }  // namespace
 
 // ============================================================ launchers ==
@@ -649,19 +584,6 @@ cudaError_t launch_mod_up_ntt(const PrimeTables &t, const DevicePartitions &dp, 
   return launch_extended_ntt(t, dp, log_n, moduli_id, ext, s, skip_own);
 }
 
-cudaError_t launch_extended_ntt(const PrimeTables &t, const DevicePartitions &dp, int log_n,
-                                int moduli_id, int64_t *ext, cudaStream_t s, bool skip_own) {
-  const long long stride = static_cast<long long>(dp.extended) << log_n;
-  PlainLoad ld{ext, stride};
-  PlainStore st{ext, stride};
-  // Value-only: the extended polynomial reaches the output only through the key
-  // inner product's reduction to [0, q) and ModDown's reduced inverse transform.
-  return forward_ntt<PlainLoad, PlainStore, kNttValueOnly>(log_n, dp.count, dp.extended, moduli_id, t,
-                                                           ld, st, ext, stride, s,
-                                                           skip_own ? dp.start : nullptr,
-                                                           skip_own ? dp.size : nullptr);
-}
-
 cudaError_t launch_key_inner_product(const PrimeTables &t, const DevicePartitions &dp, int n,
                                      int moduli_id, const int64_t *ext, const int64_t *key,
                                      int key_primes, int view_offset, int64_t *acc, cudaStream_t s,
@@ -694,18 +616,6 @@ cudaError_t launch_key_inner_product(const PrimeTables &t, const DevicePartition
   key_inner_product_kernel<<<blocks_for(static_cast<long long>(dp.extended) * n), kThreads, 0, s>>>(
       t, dp, n, moduli_id, ext, key, key_primes, view_offset, acc);
   return cudaGetLastError();
-}
-
-cudaError_t launch_mod_down_intt(const PrimeTables &t, int log_n, int moduli_id, int extended,
-                                 int64_t *acc, cudaStream_t s, int polys) {
-  if (polys < 1 || polys > 2) return cudaErrorInvalidValue;
-  const long long stride = static_cast<long long>(extended) << log_n;
-  PlainLoad ld{acc, stride};
-  EnterExitStore<true> st{acc, stride, t.n_inverse, t.q, t.k, t.exit_shoup};
-  // Value-only: the store reduces every word to [0, q).
-  return inverse_ntt<PlainLoad, EnterExitStore<true>, kNttValueOnly>(log_n, polys, extended,
-                                                                     moduli_id, t, ld, st, acc,
-                                                                     stride, s);
 }
 
 cudaError_t launch_mod_down_epilogue_ops(const PrimeTables &t, const KeySwitchTables &ks, int n,
@@ -741,102 +651,6 @@ cudaError_t launch_mod_down_epilogue(const PrimeTables &t, const KeySwitchTables
   ops.base_polys = mode == 0 ? 0 : 2;
   ops.rescale = mode == 2;
   return launch_mod_down_epilogue_ops(t, ks, n, moduli_id, limbs, acc, ops, out, s);
-}
-
-cudaError_t launch_to_ntt(const PrimeTables &t, int log_n, int polys, int limbs, int prime_base,
-                          const int64_t *x, long long x_stride, int64_t *y, long long y_stride,
-                          cudaStream_t s) {
-  EnterLoad ld{x, x_stride, t.r_squared, t.q, t.k};
-  PlainStore st{y, y_stride};
-  return forward_ntt(log_n, polys, limbs, prime_base, t, ld, st, y, y_stride, s);
-}
-
-cudaError_t launch_rescale_to_ntt(const PrimeTables &t, const KeySwitchTables &ks, int log_n,
-                                  int polys, int limbs, int src_moduli_id, const int64_t *x,
-                                  long long x_stride, int64_t *y, long long y_stride,
-                                  cudaStream_t s, const ExactLimbs &exact) {
-  const long long row = static_cast<long long>(src_moduli_id) * ks.prime_count;
-  PlainStore st{y, y_stride};
-  if (exact.poly == ExactLimbs::kAllExact) {
-    RescaleEnterLoad<false> ld{x, x_stride, ks.rescale_scale + row, ks.rescale_shoup + 2 * row,
-                               t.r_squared, t.q, t.k};
-    return forward_ntt(log_n, polys, limbs, src_moduli_id + 1, t, ld, st, y, y_stride, s);
-  }
-  RescaleEnterLoad<true> ld{x, x_stride, ks.rescale_scale + row, ks.rescale_shoup + 2 * row,
-                            t.r_squared, t.q, t.k, ks.rescale_enter_shoup + 2 * row, ks.r_mod, exact};
-  return forward_ntt<RescaleEnterLoad<true>, PlainStore, kNttMixed>(
-      log_n, polys, limbs, src_moduli_id + 1, t, ld, st, y, y_stride, s, nullptr, nullptr, exact);
-}
-
-cudaError_t launch_attach_special_ntt(const PrimeTables &t, const KeySwitchTables &ks, int log_n,
-                                      int polys, int limbs, int moduli_id, const int64_t *x,
-                                      long long x_stride, int64_t *y, long long y_stride,
-                                      cudaStream_t s) {
-  const long long n = 1LL << log_n;
-  const size_t special_bytes = static_cast<size_t>(ks.special_count) * n * sizeof(int64_t);
-  for (int p = 0; p < polys; p++) {
-    const cudaError_t e = cudaMemsetAsync(y + p * y_stride + limbs * n, 0, special_bytes, s);
-    if (e != cudaSuccess) return e;
-  }
-  ProductEnterLoad ld{x, x_stride, ks.p_product_mult_r, t.r_squared, t.q, t.k};
-  PlainStore st{y, y_stride};
-  return forward_ntt(log_n, polys, limbs, moduli_id, t, ld, st, y, y_stride, s);
-}
-
-cudaError_t launch_to_intt(const PrimeTables &t, int log_n, int polys, int limbs, int prime_base,
-                           const int64_t *x, long long x_stride, int64_t *y, long long y_stride,
-                           cudaStream_t s) {
-  PlainLoad ld{x, x_stride};
-  EnterExitStore<false> st{y, y_stride, t.n_inverse, t.q, t.k};
-  return inverse_ntt(log_n, polys, limbs, prime_base, t, ld, st, y, y_stride, s);
-}
-
-cudaError_t launch_ntt_plain(const PrimeTables &t, int log_n, int polys, int limbs, int prime_base,
-                             int64_t *x, long long stride, bool inverse, cudaStream_t s) {
-  PlainLoad ld{x, stride};
-  PlainStore st{x, stride};
-  if (inverse) return inverse_ntt(log_n, polys, limbs, prime_base, t, ld, st, x, stride, s);
-  return forward_ntt(log_n, polys, limbs, prime_base, t, ld, st, x, stride, s);
-}
-
-cudaError_t launch_tensor_to_intt(const PrimeTables &t, int log_n, int limbs, int prime_base,
-                                  const int64_t *a, const int64_t *b, int64_t *y, cudaStream_t s,
-                                  int64_t *own_ext, const DevicePartitions *dp,
-                                  const ExactLimbs &exact, bool third_only) {
-  const long long stride = static_cast<long long>(limbs) << log_n;
-  const int polys = third_only ? 1 : 3;
-  TensorLoad ld{a, b, stride, t.q, t.k};
-  ld.third_only = third_only;
-  if (own_ext != nullptr) {
-    if (dp == nullptr) return cudaErrorInvalidValue;
-    ld.own_ext = own_ext;
-    ld.part_start = dp->start;
-    ld.part_size = dp->size;
-    ld.part_count = dp->count;
-    ld.extended = dp->extended;
-  }
-  if (exact.poly == ExactLimbs::kAllExact) {
-    EnterExitStore<false> st{y, stride, t.n_inverse, t.q, t.k};
-    return inverse_ntt(log_n, polys, limbs, prime_base, t, ld, st, y, stride, s);
-  }
-  MixedExitStore st{y, stride, t.n_inverse, t.q, t.k, t.exit_shoup, exact};
-  const bool aligned = (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(b) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(y) & 15) == 0 &&
-                       (own_ext == nullptr || (reinterpret_cast<uintptr_t>(own_ext) & 15) == 0);
-  if (third_only && log_n >= 9 && aligned) {
-    // d2 first, then a plain mixed inverse transform in place.
-    note_launch();
-    tensor_third_kernel<<<blocks_for(static_cast<long long>(limbs) << (log_n - 1)), kThreads, 0, s>>>(
-        t, ld, log_n, limbs, prime_base, y);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    PlainLoad pl{y, stride};
-    return inverse_ntt<PlainLoad, MixedExitStore, kNttMixed>(log_n, 1, limbs, prime_base, t, pl, st, y,
-                                                             stride, s, exact);
-  }
-  return inverse_ntt<TensorLoad, MixedExitStore, kNttMixed>(log_n, polys, limbs, prime_base, t, ld,
-                                                            st, y, stride, s, exact);
 }
 
 }  // namespace fhe_b200

@@ -61,7 +61,6 @@ struct KeySwitchTables {
   // matter modulo q_to: (C, C') with C = rescale_scale mod q_to (q_from^-1 R, the
   // product of the two multipliers) and C' = floor(C 2^64 / q_to).
   const int64_t *rescale_enter_shoup;
-  const int64_t *r_mod;             // [P] R mod q: the rounder's 1 after the enter
   const int64_t *p_product_mult_r;  // [P] P mod q * R (zero for the special primes)
   const int64_t *p_shoup;           // [P][2] (P mod q, floor((P mod q) 2^64 / q))
   int prime_count;

@@ -12,7 +12,9 @@
 // host form of each function computes the same integers in C++.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 
 #ifdef __CUDACC__
 #define FHE_HD __host__ __device__ __forceinline__
@@ -434,22 +436,130 @@ FHE_HD int64_t rescale_word_shoup(int64_t xj, int64_t x0, int64_t rounder, uint6
   return guard(v, qs);
 }
 
+// ------------------------------------------------------------- FP64 products --
+//
+// For the scaling primes (40 and 41 bits) a word is an integer that a double holds
+// exactly, and the FP64 pipe multiplies modulo q in six instructions: with h = RN(v w)
+// and l = v w - h (one fused multiply-add, exact), qt = rint(v (w / q)) and
+//   v w - qt q = (h - qt q) + l,
+// where both steps are exact: |v w - qt q| is about q / 2, so h - qt q, an integer
+// below 2^53 in magnitude, is representable and so is the sum.  Bounds: |v| <= 2^50,
+// 0 <= w < q < 2^41: the quotient's error is 1/2 from rounding and |v| 2^-52 from w / q
+// as w times RN(1 / q), so the result lies within 3/4 q of zero, within (1/2 + 2^-6) q
+// for |v| < 2^46, and is congruent to v w modulo q.
+constexpr int kFpPrimeBits = 41;
+constexpr int kFpWordBits = kFpPrimeBits + 1;  // words a load takes as they are: below 2^42
+FHE_HD bool fp_prime(uint64_t q) {
+  return q < (uint64_t(1) << kFpPrimeBits) && q > (uint64_t(1) << 30);
+}
+
+FHE_HD double fp_fma(double a, double b, double c) {
+#ifdef __CUDA_ARCH__
+  return __fma_rn(a, b, c);
+#else
+  return std::fma(a, b, c);
+#endif
+}
+FHE_HD double fp_bits(uint64_t u) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double(static_cast<long long>(u));
+#else
+  double d;
+  std::memcpy(&d, &u, sizeof(d));
+  return d;
+#endif
+}
+FHE_HD uint64_t fp_raw(double d) {
+#ifdef __CUDA_ARCH__
+  return static_cast<uint64_t>(__double_as_longlong(d));
+#else
+  uint64_t u;
+  std::memcpy(&u, &d, sizeof(u));
+  return u;
+#endif
+}
+// The sign bit: every value below is an integer and never -0 (sums that cancel give +0).
+FHE_HD bool fp_negative(double x) {
+#ifdef __CUDA_ARCH__
+  return __double2hiint(x) < 0;
+#else
+  return (fp_raw(x) >> 63) != 0;
+#endif
+}
+constexpr double kFpWordBias = 4503599627370496.0;   // 2^52
+constexpr double kFpRound = 6755399441055744.0;      // 1.5 2^52: adding it rounds to an integer
+// Integers in [0, 2^52) and their words: the bias places the word in the mantissa.
+FHE_HD double fp_from_word(uint64_t w) { return fp_bits(w | 0x4330000000000000ull) - kFpWordBias; }
+FHE_HD int64_t fp_to_word(double x) {
+  return static_cast<int64_t>(fp_raw(x + kFpWordBias) & 0x000FFFFFFFFFFFFFull);
+}
+
+struct FpPrime {
+  double q, inv_q;
+};
+FHE_HD double fp_mul(double v, double w, double w_over_q, double q) {
+  const double h = v * w;
+  const double qt = fp_fma(v, w_over_q, kFpRound) - kFpRound;
+  const double l = fp_fma(v, w, -h);
+  return fp_fma(-qt, q, h) + l;
+}
+FHE_HD double fp_mul(double v, double w, const FpPrime &f) { return fp_mul(v, w, w * f.inv_q, f.q); }
+// x modulo q in [-q/2, q/2] (up to the quotient's error), |x| < 2^51.
+FHE_HD double fp_reduce(double x, const FpPrime &f) {
+  const double qt = fp_fma(x, f.inv_q, kFpRound) - kFpRound;
+  return fp_fma(-qt, f.q, x);
+}
+FHE_HD double fp_canonical(double r, const FpPrime &f) { return fp_negative(r) ? r + f.q : r; }
+// The word mont_mult(W, v) gives for the Montgomery word W = w R (mod q) below 2^42 and
+// v in [0, 2^42): t = (W v + s q) / R with 0 <= s < R is the representative of v w in
+// [W v / R, W v / R + q), and W v / R is below q, so t is the canonical residue r where
+// r >= W v / R and r + q elsewhere.  One fused multiply-add gives the exact sign of
+// r - W v / R (w_mont = W 2^-62).
+FHE_HD double fp_mont_mult(double v, double w, double w_over_q, double w_mont, const FpPrime &f) {
+  const double r = fp_canonical(fp_mul(v, w, w_over_q, f.q), f);
+  return fp_negative(fp_fma(-w_mont, v, r)) ? r + f.q : r;
+}
+// The word mont_exit(mont_mult(v, N^-1 R)) gives for v in [0, 2^42), r the canonical
+// residue of v N^-1 R^-1: r, but q for a non-zero v whose residue is 0 (mont_exit's result
+// lies in [t / R, t / R + q) for the product t, which is positive where v is).
+FHE_HD double fp_exit_word(double v, double r, const FpPrime &f) { return r == 0.0 && v != 0.0 ? f.q : r; }
+// A word that a load cannot take as it is (negative, or 2^42 and more), as a value
+// congruent to it below 2^42.
+FHE_HD double fp_from_any_word(int64_t w, const FpPrime &f) {
+  const double high = static_cast<double>(static_cast<int32_t>(w >> 32));
+  return fp_mul(high, 4294967296.0, 4294967296.0 * f.inv_q, f.q) +
+         fp_from_word(static_cast<uint32_t>(w));
+}
+constexpr double kFpMontScale = 1.0 / 4611686018427387904.0;  // 2^-62
+
 FHE_HD bool redc_operand_ok(int64_t x) {
   return static_cast<uint64_t>(x) < (uint64_t(1) << 61);
 }
+
+struct PrimeSet {
+  uint64_t bits[2] = {};  // primes from 128 on are not in it
+  bool has(int prime) const { return prime < 128 && ((bits[prime >> 6] >> (prime & 63)) & 1) != 0; }
+  void add(int prime) {
+    if (prime < 128) bits[prime >> 6] |= uint64_t(1) << (prime & 63);
+  }
+};
 
 // Per-prime constants as the kernels read them.
 struct PrimeTables {
   const uint64_t *q;
   const uint64_t *k;
   const int64_t *r_squared;
+  const int64_t *r_mod;         // R mod q, r_squared's plain value
   const int64_t *n_inverse;
   const int64_t *root;          // [prime][N-1]
   const int64_t *root_inverse;  // [prime][N-1]
   const int64_t *root_reduced;          // root, each word reduced to [0, q)
   const int64_t *root_inverse_reduced;  // root_inverse, each word reduced to [0, q)
   // The same twiddles as (W, W') pairs for shoup_mult: W = root R^-1 mod q, the
-  // plain twiddle, and W' = floor(W 2^64 / q); [prime][N-1][2].
+  // plain twiddle, and W' = floor(W 2^64 / q); [prime][N][2], entries 0 .. N-2.  A prime
+  // that fp_prime accepts holds two rows of N doubles there instead: W, then the Montgomery
+  // word root 2^-62 (fp_mul, fp_mont_mult); twiddle i is entry i + 1 of a forward row and
+  // entry i of an inverse one.
   const int64_t *root_shoup;
   const int64_t *root_inverse_shoup;
   // (C, C') per prime for the reduced exit of a value-only inverse transform:
@@ -458,6 +568,7 @@ struct PrimeTables {
   const int64_t *exit_shoup;
   const double *inv_q;          // 1 / q
   const double *inv_2q;         // 1 / (2q)
+  PrimeSet fp_primes;           // the primes that fp_prime accepts
   int log_n;
 };
 

@@ -19,27 +19,58 @@ inline unsigned grid_for(long long work) {
 // mont_enter(mont_enter(c0, P mod q * R), R^2) on the way into the forward NTT
 // (create_key_switcher_for_rotate, core_key_switch.cpp:550-576).
 struct ScaledEnterLoad {
+  static constexpr bool kFp = true;
+  using Raw = int64_t;
+  using Const = FpFactor;
   const int64_t *src;
   const int64_t *p_product_mult_r;  // indexed by prime
   const int64_t *r_squared;
   const uint64_t *q;
   const uint64_t *k;
-  __device__ __forceinline__ int64_t operator()(int, int limb, int prime, int gi, int n) const {
+  __device__ __forceinline__ Raw raw(int, int limb, int gi, int n) const {
+    return src[static_cast<long long>(limb) * n + gi];
+  }
+  __device__ __forceinline__ int64_t word(Raw x, int, int, int prime) const {
     const uint64_t qq = q[prime], kk = k[prime];
-    const int64_t x = src[static_cast<long long>(limb) * n + gi];
     return mont_mult_lazy(mont_mult_lazy(x, p_product_mult_r[prime], qq, kk), r_squared[prime], qq, kk);
+  }
+  // The value of both products: x times the plain residue P R.
+  __device__ __forceinline__ Const constants(int prime, const FpPrime &f) const {
+    return fp_factor(p_product_mult_r[prime], 0, f);
+  }
+  template <bool EXACT>
+  __device__ __forceinline__ bool odd(Raw x) const { return fp_odd(x); }
+  template <bool EXACT>
+  __device__ __forceinline__ double fp(Raw x, const Const &c, const FpPrime &f, bool &) const {
+    static_assert(!EXACT, "the accumulated term is read modulo q only");
+    return fp_mul(fp_small(x), c.w, c.w_over_q, f.q);
+  }
+  __device__ __forceinline__ double fp_any(Raw x, const Const &c, const FpPrime &f) const {
+    return fp_mul(fp_from_any_word(x, f), c.w, c.w_over_q, f.q);
   }
 };
 
 // dst = reduce_2q_to_q(reduce(dst + v, 2q)) (mont_add_reduce_2q_to_q on the
 // accumulator of the key product).
 struct AccumulateStore {
+  using Const = NoConst;
   int64_t *dst;
   const uint64_t *q;
-  __device__ __forceinline__ void operator()(int, int limb, int prime, int gi, int n, int64_t v) const {
+  __device__ __forceinline__ void word(int, int limb, int prime, int gi, int n, int64_t v) const {
+    add(limb, prime, gi, n, before(limb, gi, n), v);
+  }
+  __device__ __forceinline__ Const constants(int, const FpPrime &) const { return {}; }
+  __device__ __forceinline__ int64_t before(int limb, int gi, int n) const {
+    return dst[static_cast<long long>(limb) * n + gi];
+  }
+  __device__ __forceinline__ void add(int limb, int prime, int gi, int n, int64_t sum, int64_t v) const {
     const int64_t qs = static_cast<int64_t>(q[prime]);
-    int64_t *p = dst + static_cast<long long>(limb) * n + gi;
-    *p = guard(guard(*p + v, qs << 1), qs);
+    dst[static_cast<long long>(limb) * n + gi] = guard(guard(sum + v, qs << 1), qs);
+  }
+  template <bool EXACT>
+  __device__ __forceinline__ void fp(int, int limb, int prime, int gi, int n, const Const &,
+                                     const FpPrime &f, int64_t sum, double x) const {
+    add(limb, prime, gi, n, sum, fp_store_word<EXACT>(x, f));
   }
 };
 
