@@ -86,6 +86,7 @@ template <int G, int P>
 __global__ void __launch_bounds__(kBsgsThreads, G <= 4 ? 3 : 2)
 bsgs_inner_kernel(PrimeTables t, int log_n, int moduli_id, int extended, const int64_t *x,
                   long long x_stride, const int64_t *dec, const __grid_constant__ BsgsInner b) {
+  chained_kernel_begin();
   BsgsWord w;
   const int n = 1 << log_n;
   w.per_poly = static_cast<long long>(extended) << log_n;
@@ -188,7 +189,7 @@ cudaError_t launch_groups(unsigned grid, cudaStream_t s, int partitions, const P
   switch (partitions) {
 #define FHE_BSGS_CASE(P)                                                                     \
   case P:                                                                                    \
-    bsgs_inner_kernel<G, P><<<grid, kBsgsThreads, 0, s>>>(t, log_n, moduli_id, extended, x, \
+    launch_chained(bsgs_inner_kernel<G, P>, grid, kBsgsThreads, 0, s, t, log_n, moduli_id, extended, x, \
                                                           x_stride, dec, b);                 \
     break;
     FHE_BSGS_CASE(1) FHE_BSGS_CASE(2) FHE_BSGS_CASE(3) FHE_BSGS_CASE(4)

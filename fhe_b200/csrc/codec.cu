@@ -38,6 +38,7 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 // bitrev(codec - 1 - pre[index]).
 __global__ void encode_scatter_kernel(const double *re, const double *im, int slot, int log_codec,
                                       const int32_t *pre, double2 *y) {
+  chained_kernel_begin();
   const int index = blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= slot) return;
   const int codec = 1 << log_codec;
@@ -50,6 +51,7 @@ __global__ void encode_scatter_kernel(const double *re, const double *im, int sl
 
 // One radix-2 stage of fft (fft.cpp:77-102): step 2^s, twiddle stride codec >> s.
 __global__ void fft_stage_kernel(double2 *y, const double2 *twiddle, int log_codec, int s) {
+  chained_kernel_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (1 << (log_codec - 1))) return;
   const int half = 1 << (s - 1);
@@ -66,6 +68,7 @@ __global__ void fft_stage_kernel(double2 *y, const double2 *twiddle, int log_cod
 // max_absolute reduction (single.cpp:567-575) of the result.
 __global__ void encode_twist_kernel(const double2 *y, int codec, const double2 *twist, double scale,
                                     double *v, unsigned long long *max_bits) {
+  chained_kernel_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= codec) return;
   const double size = static_cast<double>(codec);
@@ -86,6 +89,7 @@ __device__ __forceinline__ int64_t positive_mod(int64_t x, int64_t m) { return (
 __global__ void encode_tile_kernel(const double *v, const unsigned long long *max_bits, PrimeTables t,
                                    int first_prime, int limbs, const int64_t *multiplier,
                                    int limb_offset, int jump, int codec, int log_n, int64_t *out) {
+  chained_kernel_begin();
   const long long w = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (w >= static_cast<long long>(limbs) * codec) return;
   const int j = static_cast<int>(w / codec);
@@ -158,6 +162,7 @@ __device__ __forceinline__ double words_to_double(const uint64_t *a, int words) 
 // residue mod Q); one limb: make_signed (unit.cpp:36-42, unsigned comparison).
 __global__ void decode_crt_kernel(const int64_t *x, PrimeTables t, int first_prime, int jump,
                                   int codec, int log_n, CrtConstants c, double *out) {
+  chained_kernel_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= codec) return;
   const long long pos = static_cast<long long>(i) * jump;
@@ -226,6 +231,7 @@ __global__ void decode_crt_kernel(const int64_t *x, PrimeTables t, int first_pri
 
 // apply_skewer (encode.cpp:292-301) and bit_reversal_permute.
 __global__ void decode_skew_kernel(const double *x, int log_codec, const double2 *skew, double2 *y) {
+  chained_kernel_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (1 << log_codec)) return;
   const double v = x[i];
@@ -235,6 +241,7 @@ __global__ void decode_skew_kernel(const double *x, int log_codec, const double2
 // permute_after_ifft (encode.cpp:481-503).
 __global__ void decode_permute_kernel(const double2 *z, int codec, int slot, const int32_t *post,
                                       double scale_inverse, double *re, double *im) {
+  chained_kernel_begin();
   const int index = blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= codec) return;
   const int p = post[index];
@@ -278,7 +285,7 @@ const Engine::DeviceCodec &Engine::codec() {
 void Engine::fft_on_device(double2 *y, const double2 *twiddle, int log_codec) {
   for (int s = 1; s <= log_codec; s++) {
     note_launch();
-    fft_stage_kernel<<<grid_for(1LL << (log_codec - 1)), kThreads, 0, stream_>>>(y, twiddle,
+    launch_chained(fft_stage_kernel, grid_for(1LL << (log_codec - 1)), kThreads, 0, stream_, y, twiddle,
                                                                                  log_codec, s);
   }
   check(cudaGetLastError(), "fft");
@@ -336,15 +343,14 @@ std::unique_ptr<Data> Engine::encode(const double *re, const double *im, int cou
   if (e == cudaSuccess)
     e = timed("encode", [&] {
       note_launch();
-      encode_scatter_kernel<<<grid_for(slot), kThreads, 0, stream_>>>(
+      launch_chained(encode_scatter_kernel, grid_for(slot), kThreads, 0, stream_, 
           d_in, im ? d_in + slot : nullptr, slot, dc.log_codec, dc.pre, y);
       fft_on_device(y, dc.fft, dc.log_codec);
       note_launch();
-      encode_twist_kernel<<<grid_for(codec_n), kThreads, 0, stream_>>>(
+      launch_chained(encode_twist_kernel, grid_for(codec_n), kThreads, 0, stream_, 
           y, codec_n, dc.twist, el.scale_before_tile, v, max_bits);
       note_launch();
-      encode_tile_kernel<<<grid_for(static_cast<long long>(limbs) * codec_n), kThreads, 0,
-                           stream_>>>(v, max_bits, tables_, el.first_moduli_id, limbs, multiplier,
+      launch_chained(encode_tile_kernel, grid_for(static_cast<long long>(limbs) * codec_n), kThreads, 0, stream_, v, max_bits, tables_, el.first_moduli_id, limbs, multiplier,
                                       limb_offset, params.n / codec_n, codec_n, params.log_n,
                                       pt->d);
       return cudaGetLastError();
@@ -457,15 +463,15 @@ void Engine::decode(const Data &pt, double *re, double *im) {
       c.modulus = d_mod;
       c.half = d_half;
       note_launch();
-      decode_crt_kernel<<<grid_for(codec_n), kThreads, 0, stream_>>>(
+      launch_chained(decode_crt_kernel, grid_for(codec_n), kThreads, 0, stream_, 
           x->d, tables_, mid, params.n / codec_n, codec_n, params.log_n, c, plain);
       note_launch();
-      decode_skew_kernel<<<grid_for(codec_n), kThreads, 0, stream_>>>(plain, dc.log_codec, dc.skew,
+      launch_chained(decode_skew_kernel, grid_for(codec_n), kThreads, 0, stream_, plain, dc.log_codec, dc.skew,
                                                                        z);
       fft_on_device(z, dc.ifft, dc.log_codec);
       const double scale_inverse = static_cast<double>(1.0 / output_scale);
       note_launch();
-      decode_permute_kernel<<<grid_for(codec_n), kThreads, 0, stream_>>>(
+      launch_chained(decode_permute_kernel, grid_for(codec_n), kThreads, 0, stream_, 
           z, codec_n, slot, dc.post, scale_inverse, d_re, im ? d_im : nullptr);
       return cudaGetLastError();
     });

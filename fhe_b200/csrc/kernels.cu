@@ -63,6 +63,7 @@ inline unsigned blocks_for(long long work) {
 
 __global__ void tensor_kernel(PrimeTables t, int n, int limbs, int prime_base, const int64_t *a,
                               const int64_t *b, int64_t *z) {
+  chained_kernel_begin();
   const long long total = static_cast<long long>(limbs) * n;
   const long long ps = total;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -79,6 +80,7 @@ __global__ void tensor_kernel(PrimeTables t, int n, int limbs, int prime_base, c
 
 __global__ void add_reduce_kernel(PrimeTables t, int n, int limbs, int prime_base, long long total,
                                   const int64_t *x1, const int64_t *x2, int64_t *y) {
+  chained_kernel_begin();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int prime = prime_base + static_cast<int>((i >> (__ffs(n) - 1)) % limbs);
@@ -92,6 +94,7 @@ __global__ void add_reduce_kernel(PrimeTables t, int n, int limbs, int prime_bas
 
 __global__ void rescale_kernel(PrimeTables t, KeySwitchTables ks, int n, int limbs, int moduli_id,
                                const int64_t *x, long long xs, int64_t *y, long long ys) {
+  chained_kernel_begin();
   const int poly = blockIdx.y;
   const long long per_poly = static_cast<long long>(limbs - 1) * n;
   // get_rounder compares the signed word with the unsigned q/2 (unit.cpp:67-70), so
@@ -122,6 +125,7 @@ constexpr int kScalarLimbsPerThread = 4;
 __global__ void scalar_rescale_kernel(PrimeTables t, KeySwitchTables ks, int log_n, int limbs,
                                       int moduli_id, LimbScalars c, const int64_t *x,
                                       long long xs, int64_t *y, long long ys) {
+  chained_kernel_begin();
   const int poly = blockIdx.z;
   const long long cidx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (cidx >= (1LL << log_n)) return;
@@ -155,6 +159,7 @@ template <int A>
 __global__ void __launch_bounds__(256, A <= 10 ? 3 : 2)
     mixed_radix_kernel(PrimeTables t, DevicePartitions dp, int n, int moduli_id,
                                    const int64_t *x, int64_t *digits) {
+  chained_kernel_begin();
   const int p = blockIdx.y;
   if (dp.size[p] != A) return;
   const int start = dp.start[p];
@@ -203,6 +208,7 @@ template <int A>
 __global__ void __launch_bounds__(256)
     mod_up_contract_kernel(PrimeTables t, DevicePartitions dp, int n, int moduli_id,
                            const int64_t *digits, int64_t *ext, bool skip_own) {
+  chained_kernel_begin();
   const int p = blockIdx.y;
   if (dp.size[p] != A) return;
   const int coeff = blockIdx.x * blockDim.x + threadIdx.x;
@@ -273,6 +279,7 @@ __global__ void __launch_bounds__(256)
 __global__ void key_inner_product_kernel(PrimeTables t, DevicePartitions dp, int n, int moduli_id,
                                          const int64_t *ext, const int64_t *key, int key_primes,
                                          int view_offset, int64_t *acc) {
+  chained_kernel_begin();
   const int E = dp.extended;
   const long long total = static_cast<long long>(E) * n;
   const int log_n = __ffs(n) - 1;
@@ -340,6 +347,7 @@ __global__ void __launch_bounds__(256, P == 3 ? 4 : 0)  // three partitions: 4 C
 key_inner_product_fixed_kernel(PrimeTables t, DevicePartitions dp, int log_n, int moduli_id,
                                const int64_t *ext, const int64_t *key, long long poly_row,
                                KeyRowOffsets rows, int64_t *acc, TensorAddend add) {
+  chained_kernel_begin();
   const long long total = static_cast<long long>(dp.extended) << log_n;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -447,6 +455,7 @@ template <int K>
 __global__ void __launch_bounds__(256)
     mod_down_epilogue_kernel(PrimeTables t, KeySwitchTables ks, int n, int moduli_id, int limbs,
                              const int64_t *acc, EpilogueOps ops, int64_t *out) {
+  chained_kernel_begin();
   constexpr int CB = kEpilogueCoeffs;
   __shared__ int64_t divisor[K][CB];
   __shared__ int64_t first_limb[CB];
@@ -502,7 +511,7 @@ __global__ void __launch_bounds__(256)
 cudaError_t launch_tensor(const PrimeTables &t, int n, int limbs, int prime_base, const int64_t *a,
                           const int64_t *b, int64_t *z, cudaStream_t s) {
   note_launch();
-  tensor_kernel<<<blocks_for(static_cast<long long>(limbs) * n), kThreads, 0, s>>>(t, n, limbs,
+  launch_chained(tensor_kernel, blocks_for(static_cast<long long>(limbs) * n), kThreads, 0, s, t, n, limbs,
                                                                                   prime_base, a, b, z);
   return cudaGetLastError();
 }
@@ -511,7 +520,7 @@ cudaError_t launch_add_reduce(const PrimeTables &t, int n, int polys, int limbs,
                               const int64_t *x1, const int64_t *x2, int64_t *y, cudaStream_t s) {
   const long long total = static_cast<long long>(polys) * limbs * n;
   note_launch();
-  add_reduce_kernel<<<blocks_for(total), kThreads, 0, s>>>(t, n, limbs, prime_base, total, x1, x2, y);
+  launch_chained(add_reduce_kernel, blocks_for(total), kThreads, 0, s, t, n, limbs, prime_base, total, x1, x2, y);
   return cudaGetLastError();
 }
 
@@ -520,7 +529,7 @@ cudaError_t launch_rescale(const PrimeTables &t, const KeySwitchTables &ks, int 
                            long long ys, cudaStream_t s) {
   const dim3 grid(blocks_for(static_cast<long long>(limbs - 1) * n), polys);
   note_launch();
-  rescale_kernel<<<grid, kThreads, 0, s>>>(t, ks, n, limbs, moduli_id, x, xs, y, ys);
+  launch_chained(rescale_kernel, grid, kThreads, 0, s, t, ks, n, limbs, moduli_id, x, xs, y, ys);
   return cudaGetLastError();
 }
 
@@ -533,7 +542,7 @@ cudaError_t launch_scalar_rescale(const PrimeTables &t, const KeySwitchTables &k
   const dim3 grid(blocks_for(n), (limbs - 1 + kScalarLimbsPerThread - 1) / kScalarLimbsPerThread,
                   polys);
   note_launch();
-  scalar_rescale_kernel<<<grid, kThreads, 0, s>>>(t, ks, log_n, limbs, moduli_id, c, x, x_stride,
+  launch_chained(scalar_rescale_kernel, grid, kThreads, 0, s, t, ks, log_n, limbs, moduli_id, c, x, x_stride,
                                                   y, y_stride);
   return cudaGetLastError();
 }
@@ -546,7 +555,7 @@ cudaError_t launch_mixed_radix(const PrimeTables &t, const DevicePartitions &dp,
     if (!(dp.size_mask & (1u << size))) continue;
     switch (size) {
 #define FHE_MRS_CASE(A) \
-  case A: note_launch(); mixed_radix_kernel<A><<<grid, kThreads, 0, s>>>(t, dp, n, moduli_id, x, digits); break;
+  case A: note_launch(); launch_chained(mixed_radix_kernel<A>, grid, kThreads, 0, s, t, dp, n, moduli_id, x, digits); break;
       FHE_MRS_CASE(1) FHE_MRS_CASE(2) FHE_MRS_CASE(3) FHE_MRS_CASE(4) FHE_MRS_CASE(5)
       FHE_MRS_CASE(6) FHE_MRS_CASE(7) FHE_MRS_CASE(8) FHE_MRS_CASE(9) FHE_MRS_CASE(10)
       FHE_MRS_CASE(11) FHE_MRS_CASE(12) FHE_MRS_CASE(13) FHE_MRS_CASE(14) FHE_MRS_CASE(15)
@@ -569,7 +578,7 @@ cudaError_t launch_mod_up_ntt(const PrimeTables &t, const DevicePartitions &dp, 
 #define FHE_MU_CASE(A)                                                                    \
   case A:                                                                                 \
     note_launch();                                                                        \
-    mod_up_contract_kernel<A><<<grid, kThreads, 0, s>>>(t, dp, n, moduli_id, digits, ext, skip_own); \
+    launch_chained(mod_up_contract_kernel<A>, grid, kThreads, 0, s, t, dp, n, moduli_id, digits, ext, skip_own); \
     break;
       FHE_MU_CASE(1) FHE_MU_CASE(2) FHE_MU_CASE(3) FHE_MU_CASE(4) FHE_MU_CASE(5)
       FHE_MU_CASE(6) FHE_MU_CASE(7) FHE_MU_CASE(8) FHE_MU_CASE(9) FHE_MU_CASE(10)
@@ -603,7 +612,7 @@ cudaError_t launch_key_inner_product(const PrimeTables &t, const DevicePartition
     switch (dp.count) {
 #define FHE_KIP_CASE(P)                                                                           \
   case P:                                                                                         \
-    key_inner_product_fixed_kernel<P><<<grid, kThreads, 0, s>>>(t, dp, log_n, moduli_id, ext, key, \
+    launch_chained(key_inner_product_fixed_kernel<P>, grid, kThreads, 0, s, t, dp, log_n, moduli_id, ext, key, \
                                                                 poly_row, rows, acc, addend);    \
     break;
       FHE_KIP_CASE(1) FHE_KIP_CASE(2) FHE_KIP_CASE(3) FHE_KIP_CASE(4)
@@ -613,7 +622,7 @@ cudaError_t launch_key_inner_product(const PrimeTables &t, const DevicePartition
     return cudaGetLastError();
   }
   note_launch();
-  key_inner_product_kernel<<<blocks_for(static_cast<long long>(dp.extended) * n), kThreads, 0, s>>>(
+  launch_chained(key_inner_product_kernel, blocks_for(static_cast<long long>(dp.extended) * n), kThreads, 0, s, 
       t, dp, n, moduli_id, ext, key, key_primes, view_offset, acc);
   return cudaGetLastError();
 }
@@ -629,7 +638,7 @@ cudaError_t launch_mod_down_epilogue_ops(const PrimeTables &t, const KeySwitchTa
 #define FHE_MD_CASE(K)                                                                      \
   case K:                                                                                   \
     note_launch();                                                                          \
-    mod_down_epilogue_kernel<K><<<grid, kThreads, 0, s>>>(t, ks, n, moduli_id, limbs, acc, ops, \
+    launch_chained(mod_down_epilogue_kernel<K>, grid, kThreads, 0, s, t, ks, n, moduli_id, limbs, acc, ops, \
                                                           out);                             \
     break;
     FHE_MD_CASE(1) FHE_MD_CASE(2) FHE_MD_CASE(3) FHE_MD_CASE(4) FHE_MD_CASE(5) FHE_MD_CASE(6)

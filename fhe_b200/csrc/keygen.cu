@@ -85,6 +85,7 @@ __device__ __forceinline__ int64_t uniform_sample(const uint32_t *w, uint64_t ma
 __global__ void rng_uniform_kernel(RngState st, unsigned long long counter0, int log_n, int rows,
                                    const uint64_t *q, int prime_base, uint64_t fixed_max,
                                    int64_t shift, int64_t *out, long long row_stride) {
+  chained_kernel_begin();
   const long long blocks_per_row = 1LL << (log_n - 2);
   const long long b = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (b >= blocks_per_row * rows) return;
@@ -101,6 +102,7 @@ __global__ void rng_uniform_kernel(RngState st, unsigned long long counter0, int
 // down the CDT tree comparing (x_high >> 1, x_low) with each node.
 __global__ void rng_gaussian_kernel(RngState st, unsigned long long counter0, int log_n,
                                     int64_t *out) {
+  chained_kernel_begin();
   const long long b = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (b >= (1LL << (log_n - 2))) return;
   uint32_t w[16];
@@ -148,6 +150,7 @@ __global__ void rng_sparse_ternary_kernel(RngState st, unsigned long long counte
 // tile_unsigned_reduce_2q_to_q (single.cpp:315-326): one signed chain onto `limbs`.
 __global__ void tile_kernel(PrimeTables t, int log_n, int limbs, int prime_base, const int64_t *x,
                             int64_t *y, long long y_stride) {
+  chained_kernel_begin();
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (i >= (static_cast<long long>(limbs) << log_n)) return;
   const int j = static_cast<int>(i >> log_n);
@@ -162,6 +165,7 @@ __global__ void tile_kernel(PrimeTables t, int log_n, int limbs, int prime_base,
 // 1085-1108).
 __global__ void signed_tile_kernel(PrimeTables t, int log_n, int limbs, int prime_base,
                                    const int64_t *x, int64_t q_src, int64_t *y, long long y_stride) {
+  chained_kernel_begin();
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (i >= (static_cast<long long>(limbs) << log_n)) return;
   const int j = static_cast<int>(i >> log_n);
@@ -211,6 +215,7 @@ template <int W>
 __global__ void pointwise_kernel(PrimeTables t, int op, int log_n, int limbs, int period,
                                  int prime_base, const int64_t *a, const int64_t *b, LimbScalars c,
                                  int64_t *y) {
+  chained_kernel_begin();
   const long long i0 = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) * W;
   if (i0 >= (static_cast<long long>(limbs) << log_n)) return;
   const int j = static_cast<int>(i0 >> log_n) % period;  // W <= N: the words share a limb
@@ -269,7 +274,7 @@ void Engine::draw_uniform(int64_t *out, long long row_stride, int rows, int prim
                           uint64_t fixed_max, int64_t shift) {
   const long long blocks = (static_cast<long long>(params.n) >> 2) * rows;
   note_launch();
-  rng_uniform_kernel<<<grid_for(blocks), kThreads, 0, stream_>>>(
+  launch_chained(rng_uniform_kernel, grid_for(blocks), kThreads, 0, stream_, 
       rng_, rng_counter_, params.log_n, rows, tables_.q, prime_base, fixed_max, shift, out,
       row_stride);
   rng_counter_ += static_cast<unsigned long long>(blocks);
@@ -280,7 +285,7 @@ void Engine::draw_gaussian(int64_t *out) {
   ensure_rng_tables();
   const long long blocks = static_cast<long long>(params.n) >> 2;
   note_launch();
-  rng_gaussian_kernel<<<grid_for(blocks), kThreads, 0, stream_>>>(rng_, rng_counter_, params.log_n,
+  launch_chained(rng_gaussian_kernel, grid_for(blocks), kThreads, 0, stream_, rng_, rng_counter_, params.log_n,
                                                                   out);
   rng_counter_ += static_cast<unsigned long long>(blocks);
   check(cudaGetLastError(), "gaussian draw");
@@ -288,7 +293,7 @@ void Engine::draw_gaussian(int64_t *out) {
 
 void Engine::tile(const int64_t *chain, int limbs, int prime_base, int64_t *y, long long y_stride) {
   note_launch();
-  tile_kernel<<<grid_for(static_cast<long long>(limbs) << params.log_n), kThreads, 0, stream_>>>(
+  launch_chained(tile_kernel, grid_for(static_cast<long long>(limbs) << params.log_n), kThreads, 0, stream_, 
       tables_, params.log_n, limbs, prime_base, chain, y, y_stride);
   check(cudaGetLastError(), "tile");
 }
@@ -296,8 +301,7 @@ void Engine::tile(const int64_t *chain, int limbs, int prime_base, int64_t *y, l
 void Engine::signed_tile(const int64_t *chain, int64_t q_src, int limbs, int prime_base,
                          int64_t *y, long long y_stride) {
   note_launch();
-  signed_tile_kernel<<<grid_for(static_cast<long long>(limbs) << params.log_n), kThreads, 0,
-                       stream_>>>(tables_, params.log_n, limbs, prime_base, chain, q_src, y,
+  launch_chained(signed_tile_kernel, grid_for(static_cast<long long>(limbs) << params.log_n), kThreads, 0, stream_, tables_, params.log_n, limbs, prime_base, chain, q_src, y,
                                   y_stride);
   check(cudaGetLastError(), "signed tile");
 }
@@ -318,10 +322,10 @@ void Engine::pointwise(int op, int limbs, int prime_base, const int64_t *a, cons
   check(timed("pointwise", [&] {
           note_launch();
           if (aligned && params.n >= 4)
-            pointwise_kernel<4><<<grid_for(words / 4), kThreads, 0, stream_>>>(
+            launch_chained(pointwise_kernel<4>, grid_for(words / 4), kThreads, 0, stream_, 
                 tables_, op, params.log_n, limbs, period, prime_base, a, b, c, y);
           else
-            pointwise_kernel<1><<<grid_for(words), kThreads, 0, stream_>>>(
+            launch_chained(pointwise_kernel<1>, grid_for(words), kThreads, 0, stream_, 
                 tables_, op, params.log_n, limbs, period, prime_base, a, b, c, y);
           return cudaGetLastError();
         }),

@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
     mod_down_tc_kernel(PrimeTables t, KeySwitchTables ks, ModDownTcTables tc, int n,
                        int moduli_id, int L, const int64_t *acc, EpilogueOps ops, int64_t *out,
                        TcStatus status) {
+  chained_kernel_begin();
   constexpr int KB = row_bytes(K);
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t *sA = smem;                   // [128 rows][KB], core matrices
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
 #pragma unroll
     for (int u = 0; u < kHalfTargets; u++) {
       const int j = round * kTcTargets + half * kHalfTargets + u;
-      xs[u] = j < L ? __ldg(x + static_cast<long long>(j) * n + row) : 0;
+      xs[u] = j < L ? x[static_cast<long long>(j) * n + row] : 0;
     }
     ok = __syncthreads_and(mbar_wait(bar, round & 1, status.wait_limit)) != 0;
     if (!ok) break;
@@ -281,7 +282,7 @@ cudaError_t launch_mod_down_epilogue_tc(const PrimeTables &t, const KeySwitchTab
       raised[KK] |= bit;                                                                        \
     }                                                                                           \
     note_launch();                                                                              \
-    mod_down_tc_kernel<KK><<<grid, kTcThreads, smem, s>>>(t, ks, tc, n, moduli_id, limbs, acc,  \
+    launch_chained(mod_down_tc_kernel<KK>, grid, kTcThreads, smem, s, t, ks, tc, n, moduli_id, limbs, acc,  \
                                                           ops, out, status);                     \
     break;
     FHE_TC_CASE(1) FHE_TC_CASE(2) FHE_TC_CASE(3) FHE_TC_CASE(4) FHE_TC_CASE(5) FHE_TC_CASE(6)

@@ -32,6 +32,7 @@ template <int A>
 __global__ void __launch_bounds__(kTcThreads, 4)
     mod_up_tc_kernel(PrimeTables t, DevicePartitions dp, ModUpTcTables tc, int n, int moduli_id,
                      const int64_t *digits, int64_t *ext, TcStatus status, bool skip_own) {
+  chained_kernel_begin();
   constexpr int KB = digit_row_bytes(A);
   const int p = blockIdx.y;
   if (dp.size[p] != A) return;  // uniform per CTA, before any barrier
@@ -215,7 +216,7 @@ cudaError_t launch_mod_up_contract_tc(const PrimeTables &t, const DevicePartitio
       raised[AA] |= bit;                                                                          \
     }                                                                                             \
     note_launch();                                                                                \
-    mod_up_tc_kernel<AA><<<grid, kTcThreads, mod_up_tc_smem(AA), s>>>(t, dp, tc, n, moduli_id,    \
+    launch_chained(mod_up_tc_kernel<AA>, grid, kTcThreads, mod_up_tc_smem(AA), s, t, dp, tc, n, moduli_id,    \
                                                                       digits, ext, status, skip_own); \
     break;
       FHE_UP_CASE(1) FHE_UP_CASE(2) FHE_UP_CASE(3) FHE_UP_CASE(4) FHE_UP_CASE(5) FHE_UP_CASE(6)

@@ -848,6 +848,7 @@ struct NttLimbOrder {
 template <int LOG_N, bool STRIDED, bool INVERSE, class Loader, class Storer, int VALUE_ONLY>
 __global__ void __launch_bounds__(kNttThreads, 6)
     ntt_pass_kernel(NttPass a, NttLimbOrder order, PrimeTables t, Loader load, Storer store) {
+  chained_kernel_begin();
   __shared__ double tile[1 << kNttFpTileLog];
   constexpr int kIntTiles = LOG_N - kNttIntTileLog, kFpTiles = LOG_N - kNttFpTileLog;
   const int integer_blocks = (order.integer_limbs * a.polys) << kIntTiles;
@@ -893,6 +894,7 @@ __global__ void __launch_bounds__(kNttThreads, 6)
 template <int LOG_N, bool STRIDED, bool INVERSE, class Loader, class Storer, int VALUE_ONLY>
 __global__ void __launch_bounds__(kNttIntThreads, 4)
     ntt_int_kernel(NttPass a, PrimeTables t, Loader load, Storer store) {
+  chained_kernel_begin();
   extern __shared__ __align__(16) int64_t tile_smem[];
   const int poly = blockIdx.y % a.polys;
   const int limb = blockIdx.y / a.polys;
@@ -950,7 +952,7 @@ cudaError_t launch_ntt_int(const NttPass &a, const PrimeTables &t, const Loader 
   }
   if (smem > static_cast<size_t>(kNttMaxSmem)) return cudaErrorInvalidValue;
   note_launch(1);
-  kernel<<<grid, kNttIntThreads, smem, stream>>>(a, t, ld, st);
+  launch_chained(kernel, grid, kNttIntThreads, smem, stream, a, t, ld, st);
   return cudaGetLastError();
 }
 
@@ -980,8 +982,7 @@ cudaError_t launch_ntt_pass(const NttPass &a, bool standard, bool integer, const
   switch (a.log_n) {
 #define FHE_NTT_CASE(L)                                                               \
   case L:                                                                             \
-    ntt_pass_kernel<L, STRIDED, INVERSE, Loader, Storer, VALUE_ONLY>                  \
-        <<<blocks, kNttThreads, 0, stream>>>(a, order, t, ld, st);                    \
+    launch_chained(ntt_pass_kernel<L, STRIDED, INVERSE, Loader, Storer, VALUE_ONLY>, blocks, kNttThreads, 0, stream, a, order, t, ld, st);                    \
     break;
     FHE_NTT_CASE(13) FHE_NTT_CASE(14) FHE_NTT_CASE(15) FHE_NTT_CASE(16) FHE_NTT_CASE(17)
 #undef FHE_NTT_CASE

@@ -78,6 +78,7 @@ struct AccumulateStore {
 __global__ void permute_signed_kernel(PrimeTables t, int log_n, int polys, int limbs,
                                       int prime_base, const int64_t *x, long long xs,
                                       const int32_t *perm, int64_t *y, long long ys) {
+  chained_kernel_begin();
   const long long per_poly = static_cast<long long>(limbs) << log_n;
   const long long total = per_poly * polys;
   const int n = 1 << log_n;
@@ -98,6 +99,7 @@ __global__ void permute_signed_kernel(PrimeTables t, int log_n, int polys, int l
 
 __global__ void permute_gather_kernel(int log_n, int polys, int limbs, const int64_t *x,
                                       long long xs, const int32_t *perm, int64_t *y, long long ys) {
+  chained_kernel_begin();
   const long long per_poly = static_cast<long long>(limbs) << log_n;
   const long long total = per_poly * polys;
   const int n = 1 << log_n;
@@ -113,6 +115,7 @@ __global__ void permute_gather_kernel(int log_n, int polys, int limbs, const int
 __global__ void scalar_enter_kernel(PrimeTables t, int log_n, int polys, int limbs, int prime_base,
                                     const int64_t *x, long long xs, int x_limb_offset,
                                     LimbScalars s, int64_t *y, long long ys) {
+  chained_kernel_begin();
   const long long per_poly = static_cast<long long>(limbs) << log_n;
   const long long total = per_poly * polys;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -130,6 +133,7 @@ __global__ void scalar_enter_kernel(PrimeTables t, int log_n, int polys, int lim
 __global__ void ntt_rotate_finish_kernel(PrimeTables t, int log_n, int limbs, int prime_base,
                                          const int64_t *x0, const int64_t *acc,
                                          const int32_t *perm, int64_t *y) {
+  chained_kernel_begin();
   const long long per_poly = static_cast<long long>(limbs) << log_n;
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (i >= 2 * per_poly) return;
@@ -149,6 +153,7 @@ template <int W>
 __global__ void diagonal_mac_kernel(PrimeTables t, int log_n, int limbs, int prime_base,
                                     MacTerms terms, long long x_stride, bool accumulate,
                                     int64_t *y, long long y_stride) {
+  chained_kernel_begin();
   const long long per_poly = static_cast<long long>(limbs) << log_n;
   const long long i = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) * W;
   if (i >= 2 * per_poly) return;
@@ -223,7 +228,7 @@ cudaError_t launch_permute_signed(const PrimeTables &t, int n, int polys, int li
   if (x == y) return cudaErrorInvalidValue;  // a scatter cannot run in place
   const int log_n = __builtin_ctz(static_cast<unsigned>(n));
   note_launch();
-  permute_signed_kernel<<<grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, s>>>(
+  launch_chained(permute_signed_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, s, 
       t, log_n, polys, limbs, prime_base, x, x_stride, signed_perm, y, y_stride);
   return cudaGetLastError();
 }
@@ -234,7 +239,7 @@ cudaError_t launch_permute_gather(int n, int polys, int limbs, const int64_t *x,
   if (x == y) return cudaErrorInvalidValue;
   const int log_n = __builtin_ctz(static_cast<unsigned>(n));
   note_launch();
-  permute_gather_kernel<<<grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, s>>>(
+  launch_chained(permute_gather_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, s, 
       log_n, polys, limbs, x, x_stride, perm, y, y_stride);
   return cudaGetLastError();
 }
@@ -246,7 +251,7 @@ cudaError_t launch_scalar_enter(const PrimeTables &t, int n, int polys, int limb
   if (limbs > kMaxScalarLimbs) return cudaErrorInvalidValue;
   const int log_n = __builtin_ctz(static_cast<unsigned>(n));
   note_launch();
-  scalar_enter_kernel<<<grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, st>>>(
+  launch_chained(scalar_enter_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, st, 
       t, log_n, polys, limbs, prime_base, x, x_stride, x_limb_offset, s, y, y_stride);
   return cudaGetLastError();
 }
@@ -255,7 +260,7 @@ cudaError_t launch_ntt_rotate_finish(const PrimeTables &t, int log_n, int limbs,
                                      const int64_t *x0, const int64_t *acc, const int32_t *perm,
                                      int64_t *y, cudaStream_t s) {
   note_launch();
-  ntt_rotate_finish_kernel<<<grid_for((2LL * limbs) << log_n), kThreads, 0, s>>>(
+  launch_chained(ntt_rotate_finish_kernel, grid_for((2LL * limbs) << log_n), kThreads, 0, s, 
       t, log_n, limbs, prime_base, x0, acc, perm, y);
   return cudaGetLastError();
 }
@@ -270,10 +275,10 @@ cudaError_t launch_diagonal_mac(const PrimeTables &t, int log_n, int limbs, int 
     bits |= reinterpret_cast<uintptr_t>(terms.x[m]) | reinterpret_cast<uintptr_t>(terms.d[m]);
   note_launch();
   if ((bits & 15) == 0 && log_n >= 1)
-    diagonal_mac_kernel<2><<<grid_for(((2LL * limbs) << log_n) / 2), kThreads, 0, s>>>(
+    launch_chained(diagonal_mac_kernel<2>, grid_for(((2LL * limbs) << log_n) / 2), kThreads, 0, s, 
         t, log_n, limbs, prime_base, terms, x_stride, accumulate, y, y_stride);
   else
-    diagonal_mac_kernel<1><<<grid_for((2LL * limbs) << log_n), kThreads, 0, s>>>(
+    launch_chained(diagonal_mac_kernel<1>, grid_for((2LL * limbs) << log_n), kThreads, 0, s, 
         t, log_n, limbs, prime_base, terms, x_stride, accumulate, y, y_stride);
   return cudaGetLastError();
 }
