@@ -33,51 +33,151 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
                       __dadd_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x)));
 }
 
-// pre_permute (encode.cpp:156-185) followed by bit_reversal_permute
-// (fft.cpp:56-75): value `index` lands at bitrev(pre[index]) and its mirror at
-// bitrev(codec - 1 - pre[index]).
-__global__ void encode_scatter_kernel(const double *re, const double *im, int slot, int log_codec,
-                                      const int32_t *pre, double2 *y) {
-  chained_kernel_begin();
-  const int index = blockIdx.x * blockDim.x + threadIdx.x;
-  if (index >= slot) return;
-  const int codec = 1 << log_codec;
-  const int p = pre[index];
-  const double r = re[index];
-  const double i = im ? im[index] : 0.0;
-  y[bit_reverse(p, log_codec)] = make_double2(r, i);
-  y[bit_reverse(codec - 1 - p, log_codec)] = make_double2(r, im ? -i : 0.0);
-}
+// The FFT of fft (fft.cpp:77-102) in one or two launches: stages 1 .. 9 on 512 adjacent
+// elements in shared memory, the others on 512 >> (log - 9) columns of stride 512, one
+// butterfly a thread and stage, every stage's twiddle loaded ahead.  One launch a stage, the
+// form before, took 2.9 us each at N = 2^14 for 0.4 us of work.  Each butterfly is the
+// reference's, so the doubles are the same whatever the schedule.  The element-wise steps
+// before and after run in the first pass's Load and the last one's Store.
+constexpr int kFftTileLog = 9;
+constexpr int kFftThreads = 1 << (kFftTileLog - 1);
 
-// One radix-2 stage of fft (fft.cpp:77-102): step 2^s, twiddle stride codec >> s.
-__global__ void fft_stage_kernel(double2 *y, const double2 *twiddle, int log_codec, int s) {
-  chained_kernel_begin();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (1 << (log_codec - 1))) return;
-  const int half = 1 << (s - 1);
-  const int j = t & (half - 1);
-  const int a = ((t >> (s - 1)) << s) + j;
-  const int b = a + half;
-  const double2 left = y[a];
-  const double2 right = cmul(twiddle[j << (log_codec - s)], y[b]);
-  y[a] = make_double2(__dadd_rn(left.x, right.x), __dadd_rn(left.y, right.y));
-  y[b] = make_double2(__dsub_rn(left.x, right.x), __dsub_rn(left.y, right.y));
-}
+struct ComplexLoad {
+  const double2 *y;
+  __device__ __forceinline__ double2 operator()(int i) const { return y[i]; }
+};
+struct ComplexStore {
+  double2 *y;
+  __device__ __forceinline__ void operator()(int i, double2 v) { y[i] = v; }
+  __device__ __forceinline__ void finish() {}
+};
+
+// pre_permute (encode.cpp:156-185) followed by bit_reversal_permute (fft.cpp:56-75):
+// element i comes from slot source[i] (its conjugate where the top bit is set); slots past
+// the message are zero.
+struct EncodeLoad {
+  const double *re;
+  const double *im;
+  int count;
+  const uint32_t *source;
+  unsigned long long *max_bits;  // cleared for the last pass
+  __device__ __forceinline__ double2 operator()(int i) const {
+    if (i == 0) *max_bits = 0;
+    const uint32_t at = source[i];
+    const int index = static_cast<int>(at & 0x7fffffffu);
+    const double r = index < count ? re[index] : 0.0;
+    if (im == nullptr) return make_double2(r, 0.0);
+    const double c = index < count ? im[index] : 0.0;
+    return make_double2(r, (at >> 31) != 0 ? -c : c);
+  }
+};
 
 // normalize (fft.cpp:47-52) and apply_twister (encode.cpp:279-290), with the
-// max_absolute reduction (single.cpp:567-575) of the result.
-__global__ void encode_twist_kernel(const double2 *y, int codec, const double2 *twist, double scale,
-                                    double *v, unsigned long long *max_bits) {
+// max_absolute reduction (single.cpp:567-575) of the result: one atomic a warp.
+struct TwistStore {
+  int codec;
+  const double2 *twist;
+  double scale;
+  double *v;
+  unsigned long long *max_bits;
+  unsigned long long most = 0;
+  __device__ __forceinline__ void operator()(int i, double2 y) {
+    const double size = static_cast<double>(codec);
+    const double re = __ddiv_rn(y.x, size);
+    const double im = __ddiv_rn(y.y, size);
+    const double2 c = twist[i];
+    const double value = __dmul_rn(__dsub_rn(__dmul_rn(re, c.x), __dmul_rn(im, c.y)), scale);
+    v[i] = value;
+    const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(fabs(value)));
+    most = bits > most ? bits : most;
+  }
+  __device__ __forceinline__ void finish() {
+    for (int d = 16; d > 0; d >>= 1) {
+      const unsigned long long other = __shfl_xor_sync(0xffffffffu, most, d);
+      most = other > most ? other : most;
+    }
+    if ((threadIdx.x & 31) == 0) atomicMax(max_bits, most);
+  }
+};
+
+// permute_after_ifft (encode.cpp:481-503).
+struct DecodeStore {
+  const int32_t *post;
+  int slot;
+  double scale_inverse;
+  double *re;
+  double *im;
+  __device__ __forceinline__ void operator()(int i, double2 z) {
+    const int p = post[i];
+    if (p < slot) {
+      re[p] = __dmul_rn(z.x, scale_inverse);
+      if (im) im[p] = __dmul_rn(z.y, scale_inverse);
+    }
+  }
+  __device__ __forceinline__ void finish() {}
+};
+
+// Stages first + 1 .. first + count (count <= 9).  first = 0: a tile of adjacent elements;
+// else first = 9 and a tile of columns.
+template <class Load, class Store>
+__global__ void __launch_bounds__(kFftThreads)
+    fft_pass_kernel(Load load, Store store, const double2 *twiddle, int log_codec, int first, int count) {
   chained_kernel_begin();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= codec) return;
-  const double size = static_cast<double>(codec);
-  const double re = __ddiv_rn(y[i].x, size);
-  const double im = __ddiv_rn(y[i].y, size);
-  const double2 c = twist[i];
-  const double value = __dmul_rn(__dsub_rn(__dmul_rn(re, c.x), __dmul_rn(im, c.y)), scale);
-  v[i] = value;
-  atomicMax(max_bits, static_cast<unsigned long long>(__double_as_longlong(fabs(value))));
+  __shared__ double2 tile[1 << kFftTileLog];
+  const int t = threadIdx.x;
+  const int elements = log_codec < kFftTileLog ? 1 << log_codec : 1 << kFftTileLog;
+  const int columns_log = first == 0 ? 0 : kFftTileLog - count;
+  const int c = t & ((1 << columns_log) - 1), p = t >> columns_log;
+  const int lo = (blockIdx.x << columns_log) + c;  // column, where first > 0
+  const bool active = 2 * t < elements;
+  double2 w[kFftTileLog];
+#pragma unroll
+  for (int st = 1; st <= kFftTileLog; st++) {
+    if (st <= count && active) {
+      const int jh = p & ((1 << (st - 1)) - 1);
+      w[st - 1] = twiddle[(first == 0 ? jh : (jh << first) + lo) << (log_codec - first - st)];
+    }
+  }
+  auto index = [&](int i) {  // of tile element i
+    return first == 0 ? (blockIdx.x << kFftTileLog) + i
+                      : ((i >> columns_log) << first) + (blockIdx.x << columns_log) +
+                            (i & ((1 << columns_log) - 1));
+  };
+  for (int i = t; i < elements; i += kFftThreads) tile[i] = load(index(i));
+#pragma unroll
+  for (int st = 1; st <= kFftTileLog; st++) {
+    if (st > count) break;
+    __syncthreads();
+    if (active) {
+      const int half = 1 << (st - 1);
+      const int a = ((((p >> (st - 1)) << st) + (p & (half - 1))) << columns_log) + c;
+      const int b = a + (half << columns_log);
+      const double2 left = tile[a];
+      const double2 right = cmul(w[st - 1], tile[b]);
+      tile[a] = make_double2(__dadd_rn(left.x, right.x), __dadd_rn(left.y, right.y));
+      tile[b] = make_double2(__dsub_rn(left.x, right.x), __dsub_rn(left.y, right.y));
+    }
+  }
+  __syncthreads();
+  for (int i = t; i < elements; i += kFftThreads) store(index(i), tile[i]);
+  store.finish();
+}
+
+// work: 2^log_codec elements between the passes.
+template <class Load, class Store>
+cudaError_t launch_fft(const Load &load, const Store &store, const double2 *twiddle, int log_codec,
+                       double2 *work, cudaStream_t s) {
+  const unsigned tiles = log_codec <= kFftTileLog ? 1 : 1u << (log_codec - kFftTileLog);
+  note_launch();
+  if (log_codec <= kFftTileLog)
+    return launch_chained(fft_pass_kernel<Load, Store>, tiles, kFftThreads, 0, s, load, store, twiddle,
+                          log_codec, 0, log_codec);
+  const cudaError_t e = launch_chained(fft_pass_kernel<Load, ComplexStore>, tiles, kFftThreads, 0, s, load,
+                                       ComplexStore{work}, twiddle, log_codec, 0, kFftTileLog);
+  if (e != cudaSuccess) return e;
+  note_launch();
+  return launch_chained(fft_pass_kernel<ComplexLoad, Store>, tiles, kFftThreads, 0, s, ComplexLoad{work},
+                        store, twiddle, log_codec, kFftTileLog, log_codec - kFftTileLog);
 }
 
 __device__ __forceinline__ int64_t positive_mod(int64_t x, int64_t m) { return (m + x % m) % m; }
@@ -87,7 +187,7 @@ __device__ __forceinline__ int64_t positive_mod(int64_t x, int64_t m) { return (
 // then mont_enter by r_mult_scale_after_tile.  Coefficient i of the codec lands
 // at i * jump (decompress_polynomial).
 __global__ void encode_tile_kernel(const double *v, const unsigned long long *max_bits, PrimeTables t,
-                                   int first_prime, int limbs, const int64_t *multiplier,
+                                   int first_prime, int limbs, LimbScalars multiplier,
                                    int limb_offset, int jump, int codec, int log_n, int64_t *out) {
   chained_kernel_begin();
   const long long w = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -120,60 +220,76 @@ __global__ void encode_tile_kernel(const double *v, const unsigned long long *ma
     const int64_t rounded = static_cast<int64_t>(r);
     y = rounded < 0 ? rounded + q : guard(rounded, q);
   }
-  y = mont_mult(y, multiplier[j], t.q[prime], t.k[prime]);
+  y = mont_mult_lazy(y, multiplier.v[j], t.q[prime], t.k[prime]);
   out[(static_cast<long long>(limb_offset + j) << log_n) + static_cast<long long>(i) * jump] = y;
-}
-
-// Constants of the CRT reconstruction (DecodeParameters, parameter/decode.cpp):
-// for limb j, inverse_r[j] = (Q/q_j)^-1 * R mod q_j and Q/q_j as `words` 64-bit
-// words; Q and floor(Q/2) likewise.
-struct CrtConstants {
-  int limbs = 0;
-  int words = 0;
-  const int64_t *inverse_r = nullptr;  // [limbs]
-  const uint64_t *cofactor = nullptr;  // [limbs][words]
-  const uint64_t *modulus = nullptr;   // [words]
-  const uint64_t *half = nullptr;      // [words]
-};
-
-__device__ __forceinline__ bool words_ge(const uint64_t *a, const uint64_t *b, int words) {
-  for (int w = words - 1; w >= 0; w--) {
-    if (a[w] != b[w]) return a[w] > b[w];
-  }
-  return true;
 }
 
 // BigInt::get_double (big_int.cpp:219-225): sum of double(word) * 2^(64 w) in
 // word order over the trimmed words (2^(64 w) overflows to infinity past w = 15).
-__device__ __forceinline__ double words_to_double(const uint64_t *a, int words) {
-  int top = words - 1;
-  while (top > 0 && a[top] == 0) top--;
+template <int W>
+__device__ __forceinline__ double words_to_double(const uint64_t (&a)[W]) {
+  int top = 0;
+#pragma unroll
+  for (int w = 0; w < W; w++)
+    if (a[w] != 0) top = w;
   double y = 0.0;
-  for (int w = 0; w <= top; w++) {
+#pragma unroll
+  for (int w = 0; w < W; w++) {
     const double scale = w < 16 ? ldexp(1.0, 64 * w) : __longlong_as_double(0x7ff0000000000000LL);
-    y = __dadd_rn(y, __dmul_rn(__ull2double_rn(a[w]), scale));
+    if (w <= top) y = __dadd_rn(y, __dmul_rn(__ull2double_rn(a[w]), scale));
   }
   return y;
+}
+
+template <int W>
+__device__ __forceinline__ bool words_ge(const uint64_t (&a)[W], const uint64_t *b) {
+  bool ge = true;
+#pragma unroll
+  for (int w = 0; w < W; w++) ge = a[w] != b[w] ? a[w] > b[w] : ge;
+  return ge;
+}
+
+// a -= m b modulo 2^(64 W).
+template <int W>
+__device__ __forceinline__ void words_subtract(uint64_t (&a)[W], const uint64_t *b, uint64_t m) {
+  uint64_t carry = 0;
+#pragma unroll
+  for (int w = 0; w < W; w++) {
+    uint64_t lo, hi;
+    mul_wide(m, b[w], lo, hi);
+    lo += carry;
+    carry = hi + (lo < carry ? 1 : 0) + (a[w] < lo ? 1 : 0);
+    a[w] -= lo;
+  }
 }
 
 // convert_plaintext_to_double after the rescale loop (core_decode.cpp:77-98):
 // make_unsigned, then the centred CRT integer as a double (rns_to_double,
 // arithmetic.cpp:169-197, whose Montgomery BigInt reduction yields the canonical
 // residue mod Q); one limb: make_signed (unit.cpp:36-42, unsigned comparison).
-__global__ void decode_crt_kernel(const int64_t *x, PrimeTables t, int first_prime, int jump,
-                                  int codec, int log_n, CrtConstants c, double *out) {
+// Then apply_skewer (encode.cpp:292-301) and bit_reversal_permute.
+//
+// The integer is sum_j d_j Q / q_j minus floor(sum_j d_j / q_j) Q.  The floor is estimated
+// in doubles, 10^-6 low (its error is below 10^-13), so that at most two subtractions of Q are
+// left.  W words in registers, the constants in shared memory; with the word count at run time
+// the integer lay in local memory: 38 us at N = 2^16 and 10 limbs.
+template <int W>
+__global__ void __launch_bounds__(kThreads)
+    decode_crt_kernel(const int64_t *x, PrimeTables t, int first_prime, int jump, int log_codec, int log_n,
+                      CrtConstants c, const double2 *skew, double2 *y) {
   chained_kernel_begin();
+  extern __shared__ uint64_t constants[];  // [limbs][W] cofactors, Q, floor(Q / 2)
+  const int words = (c.limbs + 2) * W;
+  for (int i = threadIdx.x; i < words; i += kThreads) constants[i] = c.words[i];
+  __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= codec) return;
+  if (i >= (1 << log_codec)) return;
+  const uint64_t *modulus = constants + c.limbs * W, *half = modulus + W;
   const long long pos = static_cast<long long>(i) * jump;
-  if (c.limbs == 1) {
-    const int64_t v = x[pos];
-    const uint64_t q = t.q[first_prime];
-    out[i] = static_cast<double>(static_cast<uint64_t>(v) <= (q >> 1) ? v : v - static_cast<int64_t>(q));
-    return;
-  }
-  uint64_t acc[kMaxCrtWords + 1];
-  for (int w = 0; w <= c.words; w++) acc[w] = 0;
+  uint64_t acc[W];
+#pragma unroll
+  for (int w = 0; w < W; w++) acc[w] = 0;
+  double whole = -1e-6;
   for (int j = 0; j < c.limbs; j++) {
     const int prime = first_prime + j;
     const uint64_t qu = t.q[prime];
@@ -183,71 +299,78 @@ __global__ void decode_crt_kernel(const int64_t *x, PrimeTables t, int first_pri
     int64_t d = mont_mult(v, c.inverse_r[j], qu, t.k[prime]);
     if (d < 0) d += q;
     if (d >= q) d -= q;
+    whole += static_cast<double>(d) * t.inv_q[prime];
     // acc += d * (Q / q_j)
-    const uint64_t *cof = c.cofactor + static_cast<long long>(j) * c.words;
-    unsigned long long carry = 0;
-    for (int w = 0; w < c.words; w++) {
-      const unsigned long long lo = static_cast<unsigned long long>(d) * cof[w];
-      const unsigned long long hi = __umul64hi(static_cast<unsigned long long>(d), cof[w]);
-      const unsigned long long s = acc[w] + lo;
-      unsigned long long c1 = s < lo ? 1 : 0;
-      const unsigned long long s2 = s + carry;
-      c1 += s2 < s ? 1 : 0;
-      acc[w] = s2;
-      carry = hi + c1;
+    const uint64_t *cof = constants + j * W;
+    uint64_t carry = 0;
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+      uint64_t lo, hi;
+      mul_wide(static_cast<uint64_t>(d), cof[w], lo, hi);
+      lo += carry;
+      hi += lo < carry ? 1 : 0;
+      acc[w] += lo;
+      carry = hi + (acc[w] < lo ? 1 : 0);
     }
-    acc[c.words] += carry;
   }
-  // Reduce modulo Q: the sum is below limbs * Q.
-  for (int iter = 0; iter < 4 * kMaxCrtWords; iter++) {
-    bool ge = acc[c.words] != 0;
-    if (!ge) ge = words_ge(acc, c.modulus, c.words);
-    if (!ge) break;
-    unsigned long long borrow = 0;
-    for (int w = 0; w < c.words; w++) {
-      const unsigned long long bw = c.modulus[w];
-      const unsigned long long d = acc[w] - bw - borrow;
-      borrow = (acc[w] < bw || (acc[w] == bw && borrow)) ? 1 : 0;
-      acc[w] = d;
-    }
-    acc[c.words] -= borrow;
-  }
+  words_subtract(acc, modulus, whole > 0.0 ? static_cast<uint64_t>(whole) : 0);
+  for (int iter = 0; iter < 4 * kMaxCrtWords && words_ge(acc, modulus); iter++) words_subtract(acc, modulus, 1);
   double value;
-  if (words_ge(acc, c.half, c.words)) {
-    // Q - X
-    unsigned long long borrow = 0;
-    for (int w = 0; w < c.words; w++) {
-      const unsigned long long aw = c.modulus[w], bw = acc[w];
-      const unsigned long long d = aw - bw - borrow;
-      borrow = (aw < bw || (aw == bw && borrow)) ? 1 : 0;
-      acc[w] = d;
+  if (words_ge(acc, half)) {  // Q - X
+    uint64_t rest[W];
+#pragma unroll
+    for (int w = 0; w < W; w++) rest[w] = modulus[w];
+    uint64_t borrow = 0;
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+      const uint64_t b = acc[w] + borrow;
+      borrow = (b < borrow || rest[w] < b) ? 1 : 0;
+      rest[w] -= b;
     }
-    value = -words_to_double(acc, c.words);
+    value = -words_to_double(rest);
   } else {
-    value = words_to_double(acc, c.words);
+    value = words_to_double(acc);
   }
-  out[i] = value;
+  y[bit_reverse(i, log_codec)] = make_double2(__dmul_rn(value, skew[i].x), __dmul_rn(value, skew[i].y));
 }
 
-// apply_skewer (encode.cpp:292-301) and bit_reversal_permute.
-__global__ void decode_skew_kernel(const double *x, int log_codec, const double2 *skew, double2 *y) {
+__global__ void decode_single_kernel(const int64_t *x, PrimeTables t, int prime, int jump, int log_codec,
+                                     const double2 *skew, double2 *y) {
   chained_kernel_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (1 << log_codec)) return;
-  const double v = x[i];
-  y[bit_reverse(i, log_codec)] = make_double2(__dmul_rn(v, skew[i].x), __dmul_rn(v, skew[i].y));
+  const int64_t v = x[static_cast<long long>(i) * jump];
+  const uint64_t q = t.q[prime];
+  const double value =
+      static_cast<double>(static_cast<uint64_t>(v) <= (q >> 1) ? v : v - static_cast<int64_t>(q));
+  y[bit_reverse(i, log_codec)] = make_double2(__dmul_rn(value, skew[i].x), __dmul_rn(value, skew[i].y));
 }
 
-// permute_after_ifft (encode.cpp:481-503).
-__global__ void decode_permute_kernel(const double2 *z, int codec, int slot, const int32_t *post,
-                                      double scale_inverse, double *re, double *im) {
-  chained_kernel_begin();
-  const int index = blockIdx.x * blockDim.x + threadIdx.x;
-  if (index >= codec) return;
-  const int p = post[index];
-  if (p < slot) {
-    re[p] = __dmul_rn(z[index].x, scale_inverse);
-    if (im) im[p] = __dmul_rn(z[index].y, scale_inverse);
+// The word counts that the CRT kernel is compiled for: the least that holds `words`.
+constexpr int kCrtWords[] = {3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 32, 40, 48};
+int crt_words(int words) {
+  for (int w : kCrtWords)
+    if (w >= words) return w;
+  return 0;
+}
+
+cudaError_t launch_decode_crt(const int64_t *x, const PrimeTables &t, int first_prime, int jump,
+                              int log_codec, int log_n, const CrtConstants &c, const double2 *skew,
+                              double2 *y, cudaStream_t s) {
+  const unsigned grid = grid_for(1LL << log_codec);
+  note_launch();
+  if (c.limbs == 1)
+    return launch_chained(decode_single_kernel, grid, kThreads, 0, s, x, t, first_prime, jump, log_codec, skew, y);
+  const size_t smem = static_cast<size_t>(c.limbs + 2) * c.words_per_limb * sizeof(uint64_t);
+  switch (c.words_per_limb) {
+#define FHE_CRT_CASE(W) \
+  case W: return launch_chained(decode_crt_kernel<W>, grid, kThreads, smem, s, x, t, first_prime, jump, \
+                                log_codec, log_n, c, skew, y);
+    FHE_CRT_CASE(3) FHE_CRT_CASE(4) FHE_CRT_CASE(5) FHE_CRT_CASE(6) FHE_CRT_CASE(7) FHE_CRT_CASE(8)
+    FHE_CRT_CASE(10) FHE_CRT_CASE(12) FHE_CRT_CASE(14) FHE_CRT_CASE(16) FHE_CRT_CASE(20)
+    FHE_CRT_CASE(24) FHE_CRT_CASE(32) FHE_CRT_CASE(40) FHE_CRT_CASE(48)
+#undef FHE_CRT_CASE
+    default: return cudaErrorInvalidValue;
   }
 }
 
@@ -270,25 +393,92 @@ const Engine::DeviceCodec &Engine::codec() {
     return reinterpret_cast<const double2 *>(upload_table(v));
   };
   DeviceCodec d;
-  d.pre = upload_table(h.pre);
+  while ((1 << d.log_codec) < c) d.log_codec++;
+  auto reversed = [&](int i) {
+    int r = 0;
+    for (int b = 0; b < d.log_codec; b++) r |= ((i >> b) & 1) << (d.log_codec - 1 - b);
+    return r;
+  };
+  std::vector<uint32_t> source(c, 0);
+  for (int index = 0; index < params.slot_count; index++) {
+    source[reversed(h.pre[index])] = static_cast<uint32_t>(index);
+    source[reversed(c - 1 - h.pre[index])] = static_cast<uint32_t>(index) | 0x80000000u;
+  }
+  d.source = upload_table(source);
   d.post = upload_table(h.post);
   d.fft = pairs(h.fft_cos, h.fft_sin);
   d.ifft = pairs(h.ifft_cos, h.ifft_sin);
   d.twist = pairs(h.twist_cos, h.twist_sin);
   d.skew = pairs(h.skew_cos, h.skew_sin);
-  while ((1 << d.log_codec) < c) d.log_codec++;
   d.codec = c;
   codec_ = d;
   return codec_;
 }
 
-void Engine::fft_on_device(double2 *y, const double2 *twiddle, int log_codec) {
-  for (int s = 1; s <= log_codec; s++) {
-    note_launch();
-    launch_chained(fft_stage_kernel, grid_for(1LL << (log_codec - 1)), kThreads, 0, stream_, y, twiddle,
-                                                                                 log_codec, s);
+void *Engine::staging(size_t bytes) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  check(cudaStreamIsCapturing(stream_, &capturing), "cudaStreamIsCapturing");
+  if (capturing != cudaStreamCaptureStatusNone)
+    throw CudaError("a host vector cannot be staged inside a stream capture.");
+  StagingBuffer &b = staging_[staging_next_];
+  staging_next_ = (staging_next_ + 1) % kStagingBuffers;
+  if (b.copied)
+    check(cudaEventSynchronize(b.copied), "staging buffer");
+  else
+    check(cudaEventCreateWithFlags(&b.copied, cudaEventDisableTiming), "cudaEventCreate");
+  if (b.bytes < bytes) {
+    if (b.host) cudaFreeHost(b.host);
+    b.host = nullptr;
+    b.bytes = 0;
+    check(cudaMallocHost(&b.host, bytes), "cudaMallocHost(staging)");
+    b.bytes = bytes;
   }
-  check(cudaGetLastError(), "fft");
+  staging_last_ = &b;
+  return b.host;
+}
+
+void Engine::staging_queued() {
+  check(cudaEventRecord(staging_last_->copied, stream_), "cudaEventRecord");
+}
+
+const CrtConstants &Engine::crt_constants(int mid, int limbs) {
+  const auto key = std::make_pair(mid, limbs);
+  auto it = crt_cache_.find(key);
+  if (it != crt_cache_.end()) return it->second;
+  // DecodeParameters (parameter/decode.cpp:5-60) as exact words.
+  const int W = crt_words((limbs * 61 + 63) / 64 + 1);
+  std::vector<uint64_t> words(static_cast<size_t>(limbs + 2) * W, 0);
+  std::vector<int64_t> inverse_r(limbs, 0);
+  auto mul_small = [&](uint64_t *a, uint64_t m) {
+    unsigned __int128 carry = 0;
+    for (int w = 0; w < W; w++) {
+      const unsigned __int128 p = static_cast<unsigned __int128>(a[w]) * m + carry;
+      a[w] = static_cast<uint64_t>(p);
+      carry = p >> 64;
+    }
+  };
+  uint64_t *modulus = &words[static_cast<size_t>(limbs) * W], *half = modulus + W;
+  modulus[0] = 1;
+  for (int j = 0; j < limbs; j++) mul_small(modulus, params.q[mid + j]);
+  for (int w = 0; w < W; w++) half[w] = (modulus[w] >> 1) | (w + 1 < W ? (modulus[w + 1] << 63) : 0);
+  for (int j = 0; j < limbs; j++) {
+    uint64_t *c = &words[static_cast<size_t>(j) * W];
+    c[0] = 1;
+    const int64_t qj = static_cast<int64_t>(params.q[mid + j]);
+    int64_t inv = 1;
+    for (int i = 0; i < limbs; i++) {
+      if (i == j) continue;
+      mul_small(c, params.q[mid + i]);
+      inv = mod_mul(inv, mod_invert(static_cast<int64_t>(params.q[mid + i] % qj), qj), qj);
+    }
+    inverse_r[j] = mod_mul(inv, (INT64_C(1) << 62) % qj, qj);
+  }
+  CrtConstants c;
+  c.limbs = limbs;
+  c.words_per_limb = W;
+  c.inverse_r = upload_table(inverse_r);
+  c.words = upload_table(words);
+  return crt_cache_.emplace(key, c).first->second;
 }
 
 std::unique_ptr<Data> Engine::encode(const double *re, const double *im, int count, int level,
@@ -314,46 +504,48 @@ std::unique_ptr<Data> Engine::encode(const double *re, const double *im, int cou
   const int flag = (im ? kFlagComplex : 0) | (include_special ? kFlagSpecial : 0);
   auto pt = make_data(kUnitPlaintext, flag, mid, 1, el.ckks_scale);
 
-  // The slot values padded with zeros (CKKSCore::pad); surplus values are ignored.
+  // Surplus slot values are ignored, missing ones are zeros (CKKSCore::pad).  The message
+  // goes through pinned memory: a copy from the caller's pageable memory waits for the
+  // stream.
   const int used = count < slot ? count : slot;
-  std::vector<double> host(static_cast<size_t>(slot) * (im ? 2 : 1), 0.0);
-  if (used > 0) {
-    std::memcpy(host.data(), re, sizeof(double) * used);
-    if (im) std::memcpy(host.data() + slot, im, sizeof(double) * used);
-  }
-  const size_t in_words = even(host.size());
-  const size_t scratch_words = in_words + 2 * static_cast<size_t>(codec_n) + codec_n + 2 +
-                               el.r_mult_scale_after_tile.size();
-  int64_t *scratch = alloc_words(scratch_words);
+  const size_t in_words = even(static_cast<size_t>(used) * (im ? 2 : 1));
+  int64_t *scratch = alloc_words(in_words + 2 * static_cast<size_t>(codec_n) + codec_n + 2);
   double *d_in = reinterpret_cast<double *>(scratch);
   double2 *y = reinterpret_cast<double2 *>(scratch + in_words);
   double *v = reinterpret_cast<double *>(y + codec_n);
   unsigned long long *max_bits = reinterpret_cast<unsigned long long *>(v + codec_n);
-  int64_t *multiplier = reinterpret_cast<int64_t *>(max_bits + 2);
-  // Pageable host sources: the copies have read them when the calls return.
-  cudaError_t e = cudaMemcpyAsync(d_in, host.data(), host.size() * sizeof(double),
-                                  cudaMemcpyHostToDevice, stream_);
+  cudaError_t e = cudaSuccess;
+  try {
+    if (used > 0) {
+      const size_t bytes = sizeof(double) * used;
+      char *host = static_cast<char *>(staging(2 * bytes));
+      std::memcpy(host, re, bytes);
+      if (im) std::memcpy(host + bytes, im, bytes);
+      e = cudaMemcpyAsync(d_in, host, im ? 2 * bytes : bytes, cudaMemcpyHostToDevice, stream_);
+      staging_queued();
+    }
+  } catch (...) {
+    free_words(scratch);
+    throw;
+  }
+  if (static_cast<int>(el.r_mult_scale_after_tile.size()) > kMaxScalarLimbs) e = cudaErrorInvalidValue;
+  LimbScalars multiplier{};
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(multiplier, el.r_mult_scale_after_tile.data(),
-                        el.r_mult_scale_after_tile.size() * sizeof(int64_t), cudaMemcpyHostToDevice,
-                        stream_);
-  if (e == cudaSuccess) e = cudaMemsetAsync(y, 0, sizeof(double2) * codec_n, stream_);
-  if (e == cudaSuccess) e = cudaMemsetAsync(max_bits, 0, sizeof(unsigned long long), stream_);
-  if (e == cudaSuccess) e = cudaMemsetAsync(pt->d, 0, pt->words() * sizeof(int64_t), stream_);
+    std::copy(el.r_mult_scale_after_tile.begin(), el.r_mult_scale_after_tile.end(), multiplier.v);
+  const int jump = params.n / codec_n;
+  // Words that the tile kernel leaves out: sparse slots, the first limb of one more level.
+  if (e == cudaSuccess && (jump > 1 || limbs != pt->chains))
+    e = cudaMemsetAsync(pt->d, 0, pt->words() * sizeof(int64_t), stream_);
   if (e == cudaSuccess)
     e = timed("encode", [&] {
+      const EncodeLoad load{d_in, im ? d_in + used : nullptr, used, dc.source, max_bits};
+      const TwistStore store{codec_n, dc.twist, el.scale_before_tile, v, max_bits};
+      const cudaError_t f = launch_fft(load, store, dc.fft, dc.log_codec, y, stream_);
+      if (f != cudaSuccess) return f;
       note_launch();
-      launch_chained(encode_scatter_kernel, grid_for(slot), kThreads, 0, stream_, 
-          d_in, im ? d_in + slot : nullptr, slot, dc.log_codec, dc.pre, y);
-      fft_on_device(y, dc.fft, dc.log_codec);
-      note_launch();
-      launch_chained(encode_twist_kernel, grid_for(codec_n), kThreads, 0, stream_, 
-          y, codec_n, dc.twist, el.scale_before_tile, v, max_bits);
-      note_launch();
-      launch_chained(encode_tile_kernel, grid_for(static_cast<long long>(limbs) * codec_n), kThreads, 0, stream_, v, max_bits, tables_, el.first_moduli_id, limbs, multiplier,
-                                      limb_offset, params.n / codec_n, codec_n, params.log_n,
-                                      pt->d);
-      return cudaGetLastError();
+      return launch_chained(encode_tile_kernel, grid_for(static_cast<long long>(limbs) * codec_n), kThreads,
+                            0, stream_, v, max_bits, tables_, el.first_moduli_id, limbs, multiplier,
+                            limb_offset, jump, codec_n, params.log_n, pt->d);
     });
   free_words(scratch);
   check(e, "encode");
@@ -398,90 +590,37 @@ void Engine::decode(const Data &pt, double *re, double *im) {
   const int words = limbs > 1 ? (limbs * 61 + 63) / 64 + 1 : 1;
   if (words > kMaxCrtWords) throw std::invalid_argument(fn + ": too many limbs to decode.");
 
-  // CRT constants (DecodeParameters, parameter/decode.cpp:5-60) as exact words.
-  std::vector<uint64_t> modulus(words, 0), half(words, 0), cof(static_cast<size_t>(limbs) * words, 0);
-  std::vector<int64_t> inverse_r(limbs, 0);
-  auto mul_small = [&](uint64_t *a, uint64_t m) {
-    unsigned __int128 carry = 0;
-    for (int w = 0; w < words; w++) {
-      const unsigned __int128 p = static_cast<unsigned __int128>(a[w]) * m + carry;
-      a[w] = static_cast<uint64_t>(p);
-      carry = p >> 64;
-    }
-  };
-  if (limbs > 1) {
-    modulus[0] = 1;
-    for (int j = 0; j < limbs; j++) mul_small(modulus.data(), params.q[mid + j]);
-    for (int w = 0; w < words; w++)
-      half[w] = (modulus[w] >> 1) | (w + 1 < words ? (modulus[w + 1] << 63) : 0);
-    for (int j = 0; j < limbs; j++) {
-      uint64_t *c = &cof[static_cast<size_t>(j) * words];
-      c[0] = 1;
-      const int64_t qj = static_cast<int64_t>(params.q[mid + j]);
-      int64_t inv = 1;
-      for (int i = 0; i < limbs; i++) {
-        if (i == j) continue;
-        mul_small(c, params.q[mid + i]);
-        inv = mod_mul(inv, mod_invert(static_cast<int64_t>(params.q[mid + i] % qj), qj), qj);
-      }
-      inverse_r[j] = mod_mul(inv, (INT64_C(1) << 62) % qj, qj);
-    }
+  CrtConstants single;
+  single.limbs = 1;
+  const CrtConstants &crt = limbs > 1 ? crt_constants(mid, limbs) : single;
+  const size_t out_words = static_cast<size_t>(slot) * (im ? 2 : 1);
+  int64_t *scratch = alloc_words(2 * 2 * static_cast<size_t>(codec_n) + out_words);
+  double2 *z = reinterpret_cast<double2 *>(scratch);
+  double2 *work = z + codec_n;
+  double *d_re = reinterpret_cast<double *>(work + codec_n);
+  const double scale_inverse = static_cast<double>(1.0 / output_scale);
+  cudaError_t e = timed("decode", [&] {
+    const cudaError_t f = launch_decode_crt(x->d, tables_, mid, params.n / codec_n, dc.log_codec,
+                                            params.log_n, crt, dc.skew, z, stream_);
+    if (f != cudaSuccess) return f;
+    return launch_fft(ComplexLoad{z}, DecodeStore{dc.post, slot, scale_inverse, d_re, im ? d_re + slot : nullptr},
+                      dc.ifft, dc.log_codec, work, stream_);
+  });
+  double *host = nullptr;
+  try {
+    host = static_cast<double *>(staging(out_words * sizeof(double)));
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(host, d_re, out_words * sizeof(double), cudaMemcpyDeviceToHost, stream_);
+    staging_queued();
+  } catch (...) {
+    free_words(scratch);
+    throw;
   }
-  const size_t o_cof = even(limbs);
-  const size_t o_mod = o_cof + cof.size();
-  const size_t o_half = o_mod + words;
-  const size_t o_plain = even(o_half + words);
-  const size_t o_z = o_plain + codec_n;  // codec_n is even
-  const size_t o_re = o_z + 2 * static_cast<size_t>(codec_n);
-  int64_t *scratch = alloc_words(o_re + 2 * static_cast<size_t>(slot));
-  int64_t *d_inv = scratch;
-  uint64_t *d_cof = reinterpret_cast<uint64_t *>(scratch + o_cof);
-  uint64_t *d_mod = reinterpret_cast<uint64_t *>(scratch + o_mod);
-  uint64_t *d_half = reinterpret_cast<uint64_t *>(scratch + o_half);
-  double *plain = reinterpret_cast<double *>(scratch + o_plain);
-  double2 *z = reinterpret_cast<double2 *>(scratch + o_z);
-  double *d_re = reinterpret_cast<double *>(scratch + o_re);
-  double *d_im = d_re + slot;
-  cudaError_t e = cudaMemcpyAsync(d_inv, inverse_r.data(), limbs * sizeof(int64_t),
-                                  cudaMemcpyHostToDevice, stream_);
-  if (e == cudaSuccess && limbs > 1)
-    e = cudaMemcpyAsync(d_cof, cof.data(), cof.size() * sizeof(uint64_t), cudaMemcpyHostToDevice,
-                        stream_);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_mod, modulus.data(), words * sizeof(uint64_t), cudaMemcpyHostToDevice,
-                        stream_);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(d_half, half.data(), words * sizeof(uint64_t), cudaMemcpyHostToDevice,
-                        stream_);
-  if (e == cudaSuccess)
-    e = timed("decode", [&] {
-      CrtConstants c;
-      c.limbs = limbs;
-      c.words = words;
-      c.inverse_r = d_inv;
-      c.cofactor = d_cof;
-      c.modulus = d_mod;
-      c.half = d_half;
-      note_launch();
-      launch_chained(decode_crt_kernel, grid_for(codec_n), kThreads, 0, stream_, 
-          x->d, tables_, mid, params.n / codec_n, codec_n, params.log_n, c, plain);
-      note_launch();
-      launch_chained(decode_skew_kernel, grid_for(codec_n), kThreads, 0, stream_, plain, dc.log_codec, dc.skew,
-                                                                       z);
-      fft_on_device(z, dc.ifft, dc.log_codec);
-      const double scale_inverse = static_cast<double>(1.0 / output_scale);
-      note_launch();
-      launch_chained(decode_permute_kernel, grid_for(codec_n), kThreads, 0, stream_, 
-          z, codec_n, slot, dc.post, scale_inverse, d_re, im ? d_im : nullptr);
-      return cudaGetLastError();
-    });
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(re, d_re, slot * sizeof(double), cudaMemcpyDeviceToHost, stream_);
-  if (e == cudaSuccess && im)
-    e = cudaMemcpyAsync(im, d_im, slot * sizeof(double), cudaMemcpyDeviceToHost, stream_);
   free_words(scratch);
   check(e, "decode");
   synchronize();
+  std::memcpy(re, host, static_cast<size_t>(slot) * sizeof(double));
+  if (im) std::memcpy(im, host + slot, static_cast<size_t>(slot) * sizeof(double));
 }
 
 }  // namespace fhe_b200

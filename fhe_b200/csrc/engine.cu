@@ -65,8 +65,8 @@ Engine::Engine(const Config &config) : params(config) {
   check(cudaEventCreateWithFlags(&upload_done_, cudaEventDisableTiming), "cudaEventCreate");
   check(cudaEventCreateWithFlags(&compute_done_, cudaEventDisableTiming), "cudaEventCreate");
   set_concurrency(concurrency_);
-  check(cudaMalloc(&device_error_, sizeof(int)), "cudaMalloc(error flag)");
-  check(cudaMemset(device_error_, 0, sizeof(int)), "clear error flag");
+  check(cudaHostAlloc(&device_error_, sizeof(int), cudaHostAllocMapped), "cudaHostAlloc(error flag)");
+  *device_error_ = 0;
   // Keep freed blocks in the stream-ordered pool: key switching allocates and frees
   // the same temporaries every call.
   cudaMemPool_t pool;
@@ -253,7 +253,11 @@ Engine::~Engine() {
   for (auto &kv : signed_perm_cache_) cudaFree(kv.second);
   for (auto &kv : ntt_perm_cache_) cudaFree(kv.second);
   for (auto *b : table_buffers_) cudaFree(b);
-  if (device_error_) cudaFree(device_error_);
+  if (device_error_) cudaFreeHost(device_error_);
+  for (auto &b : staging_) {
+    if (b.host) cudaFreeHost(b.host);
+    if (b.copied) cudaEventDestroy(b.copied);
+  }
   for (auto w : workers_) {
     cudaStreamSynchronize(w);
     cudaStreamDestroy(w);
@@ -271,10 +275,9 @@ void Engine::synchronize() {
   check(cudaStreamSynchronize(upload_stream_), "cudaStreamSynchronize");
   check(cudaStreamSynchronize(download_stream_), "cudaStreamSynchronize");
   check(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
-  int flag = 0;
-  check(cudaMemcpy(&flag, device_error_, sizeof(int), cudaMemcpyDeviceToHost), "read error flag");
-  if (flag) {
-    check(cudaMemset(device_error_, 0, sizeof(int)), "clear error flag");
+  volatile int *flag = device_error_;
+  if (*flag != 0) {
+    *flag = 0;
     throw CudaError("a tensor-core wait ran out; the results since the last check are unspecified");
   }
 }

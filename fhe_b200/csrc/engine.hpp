@@ -57,6 +57,16 @@ class CudaError : public std::runtime_error {
   explicit CudaError(const std::string &what) : std::runtime_error(what) {}
 };
 
+// Constants of decode's CRT reconstruction over `limbs` limbs on the device: for limb j,
+// inverse_r[j] = (Q / q_j)^-1 R mod q_j; words holds Q / q_j per limb, Q and floor(Q / 2),
+// each of words_per_limb 64-bit words.
+struct CrtConstants {
+  int limbs = 0;
+  int words_per_limb = 0;
+  const int64_t *inverse_r = nullptr;
+  const uint64_t *words = nullptr;
+};
+
 class Engine;
 
 // Element-wise operations of Engine::pointwise over [limbs][N] views.
@@ -401,7 +411,9 @@ class Engine {
   // ModUp of every partition's digits into NTT-form extended limbs, in the selected form.
   cudaError_t mod_up(const DevicePartitions &dp, int moduli_id, const int64_t *digits,
                      int64_t *ext, bool skip_own = false);
-  int *device_error_ = nullptr;  // set by a kernel whose bounded wait ran out
+  // Set by a kernel whose bounded wait ran out.  Pinned host memory that the device writes,
+  // so that a synchronize reads it without a copy.
+  int *device_error_ = nullptr;
   uint32_t tc_wait_limit_ = kTcDefaultWaitLimit;
   TcNttTables tc_ntt_{};  // set when the ring degree has a tensor-core NTT
   // The value-only transforms run on the tensor pipe only when the tensor cores are
@@ -538,7 +550,7 @@ class Engine {
   struct DeviceCodec {
     int codec = 0;
     int log_codec = 0;
-    const int32_t *pre = nullptr;
+    const uint32_t *source = nullptr;  // slot behind element i of encode's FFT (EncodeLoad)
     const int32_t *post = nullptr;
     const double2 *fft = nullptr;    // (cos, sin) of the forward twiddles
     const double2 *ifft = nullptr;
@@ -547,7 +559,22 @@ class Engine {
   };
   DeviceCodec codec_;
   const DeviceCodec &codec();
-  void fft_on_device(double2 *y, const double2 *twiddle, int log_codec);
+  std::map<std::pair<int, int>, CrtConstants> crt_cache_;  // (first prime, limbs)
+  const CrtConstants &crt_constants(int mid, int limbs);
+  // Pinned memory for host vectors on their way to or from the device: a ring of buffers,
+  // each grown to the largest vector it carried and free again once its copy has run.
+  // staging() gives the next one, staging_queued() follows the copy's launch.
+  struct StagingBuffer {
+    void *host = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t copied = nullptr;
+  };
+  static constexpr int kStagingBuffers = 4;
+  StagingBuffer staging_[kStagingBuffers];
+  StagingBuffer *staging_last_ = nullptr;
+  int staging_next_ = 0;
+  void *staging(size_t bytes);
+  void staging_queued();
 
   // Core steps.
   std::unique_ptr<Data> core_rescale(const Data &ct);          // coefficient form

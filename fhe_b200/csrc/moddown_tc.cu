@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   if (!ok) {
     // The round's MMAs may still be running: wait for them (bounded) before the
     // tensor memory is given back.
-    if (tid == 0) atomicExch(status.error, 1);
+    if (tid == 0) *static_cast<volatile int *>(status.error) = 1;
     if (warp == 0) mbar_wait(bar, round & 1);
   }
   tc_fence_before();

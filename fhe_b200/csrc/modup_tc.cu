@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kTcThreads, 4)
     tc_fence_after();
   }
   if (!ok) {
-    if (tid == 0) atomicExch(status.error, 1);
+    if (tid == 0) *static_cast<volatile int *>(status.error) = 1;
     if (warp == 0) mbar_wait(bar, round & 1);
   }
   tc_fence_before();

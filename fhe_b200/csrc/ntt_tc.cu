@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kTcThreads, kCtasPerSm)
   if (!ok) {
     // The MMAs of the step that timed out may still run: wait for them (bounded)
     // before the tensor memory is given back.
-    if (tid == 0) atomicExch(status.error, 1);
+    if (tid == 0) *static_cast<volatile int *>(status.error) = 1;
     if (warp == 0) mbar_wait(bar, phase);
   }
   tc_fence_before();
