@@ -143,6 +143,17 @@ static void require_add_operands(const std::string &fn, const Data &a, const Dat
                              "s does not match.");
 }
 
+void Engine::pointwise_polys(int op, int polys, const Data &a, const Data &b, int64_t *y, long long ys) {
+  // Texts of the same limbs lie alike: one launch for all polynomials.
+  if (a.chains == b.chains && ys == a.poly_stride()) {
+    pointwise(op, polys * a.chains, a.moduli_id, a.d, b.d, nullptr, y, a.chains);
+    return;
+  }
+  for (int p = 0; p < polys; p++)
+    pointwise(op, a.chains, a.moduli_id, a.d + p * a.poly_stride(), b.d + p * b.poly_stride(), nullptr,
+              y + p * ys);
+}
+
 std::unique_ptr<Data> Engine::add(const Data &x, const Data &y) {
   require_add_operands("Add Unit Ciphertexts", x, y);
   Matched m = match_texts(x, y, false);
@@ -150,15 +161,11 @@ std::unique_ptr<Data> Engine::add(const Data &x, const Data &y) {
   if (a->polys < b->polys) std::swap(a, b);  // add_trio_and_duo(trio, duo), engine_add.cpp:93-100
   auto out = make_data(kUnitCiphertext, a->flag | b->flag, a->moduli_id, a->polys, a->scale);
   const long long ps = a->poly_stride();
-  for (int p = 0; p < a->polys; p++) {
-    if (p < b->polys)
-      pointwise(kOpAddReduce, a->chains, a->moduli_id, a->d + p * ps, b->d + p * b->poly_stride(),
-                nullptr, out->d + p * ps);
-    else
-      check(cudaMemcpyAsync(out->d + p * ps, a->d + p * ps, ps * sizeof(int64_t),
-                            cudaMemcpyDeviceToDevice, stream_),
-            "copy");
-  }
+  pointwise_polys(kOpAddReduce, b->polys, *a, *b, out->d, ps);
+  if (a->polys > b->polys)
+    check(cudaMemcpyAsync(out->d + b->polys * ps, a->d + b->polys * ps,
+                          (a->polys - b->polys) * ps * sizeof(int64_t), cudaMemcpyDeviceToDevice, stream_),
+          "copy");
   return out;
 }
 
@@ -172,12 +179,11 @@ std::unique_ptr<Data> Engine::subtract(const Data &x, const Data &y) {
                        a->polys >= b->polys ? a->scale : b->scale);
   const long long ps = out->poly_stride();
   const int L = out->chains, mid = out->moduli_id;
-  for (int p = 0; p < polys; p++) {
+  const int common = std::min(a->polys, b->polys);
+  pointwise_polys(kOpSubReduce, common, *a, *b, out->d, ps);
+  for (int p = common; p < polys; p++) {
     int64_t *o = out->d + p * ps;
-    if (p < a->polys && p < b->polys) {
-      pointwise(kOpSubReduce, L, mid, a->d + p * a->poly_stride(), b->d + p * b->poly_stride(),
-                nullptr, o);
-    } else if (p < a->polys) {  // subtract_trio_by_duo: third polynomial copied
+    if (p < a->polys) {  // subtract_trio_by_duo: third polynomial copied
       check(cudaMemcpyAsync(o, a->d + p * a->poly_stride(), ps * sizeof(int64_t),
                             cudaMemcpyDeviceToDevice, stream_),
             "copy");
@@ -283,9 +289,7 @@ std::unique_ptr<Data> Engine::multiply_plain(const Data &ct, const Data &pt) {
   auto p = prepare_for_multiply(pt, level);
   auto out = make_data(kUnitCiphertext, (c->flag | p->flag) & ~kFlagRescaled, c->moduli_id,
                        c->polys, c->scale * p->scale);
-  const long long ps = c->poly_stride();
-  for (int q = 0; q < c->polys; q++)
-    pointwise(kOpMult, c->chains, c->moduli_id, c->d + q * ps, p->d, nullptr, out->d + q * ps);
+  multiply_polys(c->polys, c->chains, c->moduli_id, c->d, c->poly_stride(), p->d, out->d, out->poly_stride());
   return out;
 }
 
@@ -343,10 +347,7 @@ std::unique_ptr<Data> Engine::multiply_integer(const Data &ct, int64_t value) {
   for (int j = 0; j < x->chains; j++)
     mult[j] = mod_mul(value, INT64_C(1) << 62, static_cast<int64_t>(params.q[x->moduli_id + j]));
   auto out = make_data(kUnitCiphertext, x->flag, x->moduli_id, x->polys, x->scale);
-  const long long ps = x->poly_stride();
-  for (int q = 0; q < x->polys; q++)
-    pointwise(kOpEnterReduce, x->chains, x->moduli_id, x->d + q * ps, nullptr, mult.data(),
-              out->d + q * ps);
+  pointwise(kOpEnterReduce, x->polys * x->chains, x->moduli_id, x->d, nullptr, mult.data(), out->d, x->chains);
   return out;
 }
 
@@ -356,16 +357,13 @@ std::unique_ptr<Data> Engine::negate(const Data &ct) {
     throw std::runtime_error("Negate Unit Ciphertext: the input unit ciphertext should have "
                              "either 2 or 3 polynomials.");
   auto out = make_data(ct.type, ct.flag, ct.moduli_id, ct.polys, ct.scale);
-  const long long ps = ct.poly_stride();
-  const int L = params.chains(ct.moduli_id);
-  for (int q = 0; q < ct.polys; q++) {
-    const int64_t *src = ct.d + q * ps;
-    if (ct.is_ntt()) {
-      pointwise(kOpReduce, L, ct.moduli_id, src, nullptr, nullptr, out->d + q * ps);
-      src = out->d + q * ps;
-    }
-    pointwise(kOpNegate, L, ct.moduli_id, src, nullptr, nullptr, out->d + q * ps);
+  const int L = ct.chains;
+  const int64_t *src = ct.d;
+  if (ct.is_ntt()) {
+    pointwise(kOpReduce, ct.polys * L, ct.moduli_id, src, nullptr, nullptr, out->d, L);
+    src = out->d;
   }
+  pointwise(kOpNegate, ct.polys * L, ct.moduli_id, src, nullptr, nullptr, out->d, L);
   return out;
 }
 

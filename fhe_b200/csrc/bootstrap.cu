@@ -178,10 +178,7 @@ using Owned = std::unique_ptr<Data>;
 
 void Engine::add_inplace(Data &a, const Data &b) {
   // CKKSCore::add_inplace (core.cpp:498-512): polynomial-wise reduce(a + b).
-  const long long ps = a.poly_stride();
-  for (int p = 0; p < a.polys; p++)
-    pointwise(kOpAddReduce, a.chains, a.moduli_id, a.d + p * ps, b.d + p * b.poly_stride(), nullptr,
-              a.d + p * ps);
+  pointwise_polys(kOpAddReduce, a.polys, a, b, a.d, a.poly_stride());
 }
 
 std::unique_ptr<Data> Engine::multiply_imaginary(const Data &ct, int64_t value) {
@@ -201,9 +198,7 @@ std::unique_ptr<Data> Engine::multiply_imaginary(const Data &ct, int64_t value) 
   ntt_in_place(pt->d, L, mid, pt->poly_stride(), 1);
   auto out = make_data(kUnitCiphertext, (x->flag | kFlagComplex) & ~kFlagRescaled, mid, x->polys,
                        x->scale);
-  const long long ps = x->poly_stride();
-  for (int p = 0; p < x->polys; p++)
-    pointwise(kOpMult, x->chains, mid, x->d + p * ps, pt->d, nullptr, out->d + p * ps);
+  multiply_polys(x->polys, x->chains, mid, x->d, x->poly_stride(), pt->d, out->d, out->poly_stride());
   if (!ct.is_ntt()) return to_intt(*out);
   return out;
 }
@@ -322,10 +317,8 @@ std::unique_ptr<Data> Engine::apply_butterfly(const Data &ct, bool to_slot, int 
       auto c = prepare_for_multiply(*rotated[i], level);
       auto product = make_data(kUnitCiphertext, (c->flag | p.flag) & ~kFlagRescaled, c->moduli_id,
                                c->polys, c->scale * p.scale);
-      const long long ps = c->poly_stride();
-      for (int q = 0; q < c->polys; q++)
-        pointwise(kOpMult, c->chains, c->moduli_id, c->d + q * ps, p.d, nullptr,
-                  product->d + q * ps);
+      multiply_polys(c->polys, c->chains, c->moduli_id, c->d, c->poly_stride(), p.d, product->d,
+                     product->poly_stride());
       if (!inner_sum)
         inner_sum = std::move(product);
       else

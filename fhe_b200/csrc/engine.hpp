@@ -79,6 +79,7 @@ enum PointwiseOp : int {
   kOpNegate = 5,          // negate_make_unsigned: q - a
   kOpAddScalarFirst = 6,  // add_scalar (c[limb] on coefficient 0) then reduce_2q_to_q
   kOpEnterReduce = 7,     // mont_enter(a, c[limb]) then reduce_2q_to_q
+  kOpMultReduce = 9,      // mont_mult(a, b) then reduce_2q_to_q
   kOpMonomial = 8,        // c[limb] X^(N/2), signed c tiled per limb (encode_imaginary)
 };
 
@@ -439,7 +440,14 @@ class Engine {
   void ensure_rng_tables();
   void draw_uniform(int64_t *out, long long row_stride, int rows, int prime_base, uint64_t fixed_max,
                     int64_t shift);
-  void draw_gaussian(int64_t *out);
+  void draw_gaussian(int64_t *out, int rows = 1, int uniform_bit_rows = 0);
+  // op over the first `polys` polynomials of two texts of the same level.
+  void pointwise_polys(int op, int polys, const Data &a, const Data &b, int64_t *y, long long ys);
+  // y[p] = x[p] d (Montgomery products) over the polynomials of a text.
+  void multiply_polys(int polys, int limbs, int prime_base, const int64_t *x, long long x_stride,
+                      const int64_t *d, int64_t *y, long long y_stride);
+  void encrypt_finish(int polys, int limbs, int prime_base, bool subtract, const int64_t *errors,
+                      const int64_t *plain, int64_t *ct);
   void tile(const int64_t *chain, int limbs, int prime_base, int64_t *y, long long y_stride);
   // constants: host array of `limbs` per-limb values (or null), passed by value;
   // limb j runs modulo prime prime_base + j % period (period 0: limbs).

@@ -100,30 +100,37 @@ __global__ void rng_uniform_kernel(RngState st, unsigned long long counter0, int
 
 // discrete_gaussian (random.cpp:133-170): sign bit from the high word, then a walk
 // down the CDT tree comparing (x_high >> 1, x_low) with each node.
-__global__ void rng_gaussian_kernel(RngState st, unsigned long long counter0, int log_n,
-                                    int64_t *out) {
-  chained_kernel_begin();
-  const long long b = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (b >= (1LL << (log_n - 2))) return;
-  uint32_t w[16];
-  chacha_block(st, counter0 + static_cast<unsigned long long>(b), w);
-  for (int lane = 0; lane < 4; lane++) {
-    const uint32_t *l = w + 4 * lane;
-    const uint64_t x_low = (static_cast<uint64_t>(l[0]) << 32) | l[1];
-    uint64_t x_high = (static_cast<uint64_t>(l[2]) << 32) | l[3];
-    const int64_t sign_bit = static_cast<int64_t>(x_high & 1);
-    x_high >>= 1;
-    int jump = 1, current = 0, counter = 0;
-    for (int depth = 0; depth < kCdtDepth; depth++) {
-      const uint64_t th = c_cdt[counter + current + kCdtSize];
-      const uint64_t tl = c_cdt[counter + current];
-      const int ge = (x_high > th) || (x_high == th && x_low >= tl);
-      current = 2 * current + ge;
-      counter += jump;
-      jump *= 2;
-    }
-    out[4 * b + lane] = (sign_bit * 2 - 1) * static_cast<int64_t>(current);
+__device__ __forceinline__ int64_t gaussian_sample(const uint32_t *l) {
+  const uint64_t x_low = (static_cast<uint64_t>(l[0]) << 32) | l[1];
+  uint64_t x_high = (static_cast<uint64_t>(l[2]) << 32) | l[3];
+  const int64_t sign_bit = static_cast<int64_t>(x_high & 1);
+  x_high >>= 1;
+  int jump = 1, current = 0, counter = 0;
+  for (int depth = 0; depth < kCdtDepth; depth++) {
+    const uint64_t th = c_cdt[counter + current + kCdtSize];
+    const uint64_t tl = c_cdt[counter + current];
+    const int ge = (x_high > th) || (x_high == th && x_low >= tl);
+    current = 2 * current + ge;
+    counter += jump;
+    jump *= 2;
   }
+  return (sign_bit * 2 - 1) * static_cast<int64_t>(current);
+}
+
+// grid.y consecutive draws of N samples each: Gaussian ones, then uniform bits (the random
+// polynomial of a public-key encryption).
+__global__ void rng_gaussian_kernel(RngState st, unsigned long long counter0, int log_n,
+                                    int gaussian_rows, int64_t *out) {
+  chained_kernel_begin();
+  const long long blocks = 1LL << (log_n - 2);
+  const long long b = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  if (b >= blocks) return;
+  const int row = blockIdx.y;
+  uint32_t w[16];
+  chacha_block(st, counter0 + static_cast<unsigned long long>(row * blocks + b), w);
+  int64_t *o = out + (static_cast<long long>(row) << log_n) + 4 * b;
+  for (int lane = 0; lane < 4; lane++)
+    o[lane] = row < gaussian_rows ? gaussian_sample(w + 4 * lane) : uniform_sample(w + 4 * lane, 2, 0);
 }
 
 // assign_sparse_ternary_chain (random_number_generator.cpp:62-92): hamming_weight + 1
@@ -184,6 +191,7 @@ __device__ __forceinline__ int64_t pointwise_word(int op, long long i, int log_n
   int64_t v = 0;
   switch (op) {
     case kOpMult: v = mont_mult_lazy(ai, bi, q, k); break;
+    case kOpMultReduce: v = guard(mont_mult_lazy(ai, bi, q, k), qs); break;
     case kOpAddReduce: v = guard(guard(ai + bi, q2), qs); break;
     case kOpSubReduce: v = guard(guard(ai + q2 - bi, q2), qs); break;
     case kOpReduce: v = guard(ai, qs); break;
@@ -202,7 +210,7 @@ __device__ __forceinline__ int64_t pointwise_word(int op, long long i, int log_n
 
 __device__ __forceinline__ bool pointwise_reads_a(int op) { return op != kOpMonomial; }
 __device__ __forceinline__ bool pointwise_reads_b(int op) {
-  return op == kOpMult || op == kOpAddReduce || op == kOpSubReduce;
+  return op == kOpMult || op == kOpAddReduce || op == kOpSubReduce || op == kOpMultReduce;
 }
 
 // y[j] = op(a[j], b[j]) over `limbs` limbs of N words; a, b, y are [limbs][N]
@@ -247,6 +255,63 @@ __global__ void pointwise_kernel(PrimeTables t, int op, int log_n, int limbs, in
   }
 }
 
+// y[p] = mont_mult(x[p], d) for the `polys` polynomials of a text and one of a plaintext (or
+// of a key's text and a random polynomial): d is read once for all of them.
+template <int W>
+__global__ void multiply_polys_kernel(PrimeTables t, int log_n, int limbs, int prime_base, int polys,
+                                      const int64_t *x, long long xs, const int64_t *d, int64_t *y,
+                                      long long ys) {
+  chained_kernel_begin();
+  const long long i0 = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) * W;
+  if (i0 >= (static_cast<long long>(limbs) << log_n)) return;
+  const int prime = prime_base + static_cast<int>(i0 >> log_n);  // W <= N: the words share a limb
+  const uint64_t q = t.q[prime], k = t.k[prime];
+  int64_t dv[W];
+#pragma unroll
+  for (int w = 0; w < W; w += 2) {
+    if (W > 1) {
+      const longlong2 v = *reinterpret_cast<const longlong2 *>(d + i0 + w);
+      dv[w] = v.x;
+      dv[(w + 1) % W] = v.y;
+    } else {
+      dv[w] = d[i0];
+    }
+  }
+  for (int p = 0; p < polys; p++) {
+#pragma unroll
+    for (int w = 0; w < W; w += 2) {
+      if (W > 1) {
+        const longlong2 v = *reinterpret_cast<const longlong2 *>(x + p * xs + i0 + w);
+        *reinterpret_cast<longlong2 *>(y + p * ys + i0 + w) =
+            make_longlong2(mont_mult_lazy(v.x, dv[w], q, k), mont_mult_lazy(v.y, dv[(w + 1) % W], q, k));
+      } else {
+        y[p * ys + i0] = mont_mult_lazy(x[p * xs + i0], dv[w], q, k);
+      }
+    }
+  }
+}
+
+// The errors of an encryption joined to its products: tile_unsigned_reduce_2q_to_q of the
+// sampled chains, the plaintext added to the first, then polynomial p of the text (from the
+// inverse transform) added to (or, `subtract`, taken from) error p; polys is 2, or 1 for
+// the first polynomial alone.
+__global__ void encrypt_finish_kernel(PrimeTables t, int log_n, int limbs, int prime_base, int polys,
+                                      bool subtract, const int64_t *errors, const int64_t *plain,
+                                      int64_t *ct) {
+  chained_kernel_begin();
+  const long long per_poly = static_cast<long long>(limbs) << log_n;
+  const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  if (i >= polys * per_poly) return;
+  const int poly = i >= per_poly ? 1 : 0;
+  const long long r = i - poly * per_poly;
+  const int c = static_cast<int>(r & ((1LL << log_n) - 1));
+  const int64_t q = static_cast<int64_t>(t.q[prime_base + static_cast<int>(r >> log_n)]), q2 = q << 1;
+  const int64_t v = errors[(static_cast<long long>(poly) << log_n) + c];
+  int64_t e = v < 0 ? v + q : guard(v, q);
+  if (poly == 0) e = guard(guard(plain[r] + e, q2), q);
+  ct[i] = subtract ? guard(guard(e + q2 - ct[i], q2), q) : guard(guard(ct[i] + e, q2), q);
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ host --
@@ -281,14 +346,42 @@ void Engine::draw_uniform(int64_t *out, long long row_stride, int rows, int prim
   check(cudaGetLastError(), "random draw");
 }
 
-void Engine::draw_gaussian(int64_t *out) {
+void Engine::draw_gaussian(int64_t *out, int rows, int uniform_bit_rows) {
   ensure_rng_tables();
   const long long blocks = static_cast<long long>(params.n) >> 2;
+  const dim3 grid(grid_for(blocks), rows + uniform_bit_rows);
   note_launch();
-  launch_chained(rng_gaussian_kernel, grid_for(blocks), kThreads, 0, stream_, rng_, rng_counter_, params.log_n,
-                                                                  out);
-  rng_counter_ += static_cast<unsigned long long>(blocks);
+  launch_chained(rng_gaussian_kernel, grid, kThreads, 0, stream_, rng_, rng_counter_, params.log_n, rows, out);
+  rng_counter_ += static_cast<unsigned long long>(blocks) * grid.y;
   check(cudaGetLastError(), "gaussian draw");
+}
+
+void Engine::multiply_polys(int polys, int limbs, int prime_base, const int64_t *x, long long x_stride,
+                            const int64_t *d, int64_t *y, long long y_stride) {
+  const long long words = static_cast<long long>(limbs) << params.log_n;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(d) |
+                         reinterpret_cast<uintptr_t>(y) | static_cast<uintptr_t>(x_stride * 8) |
+                         static_cast<uintptr_t>(y_stride * 8)) & 15) == 0;
+  check(timed("pointwise", [&] {
+          note_launch();
+          if (aligned && params.n >= 4)
+            launch_chained(multiply_polys_kernel<2>, grid_for(words / 2), kThreads, 0, stream_, tables_,
+                           params.log_n, limbs, prime_base, polys, x, x_stride, d, y, y_stride);
+          else
+            launch_chained(multiply_polys_kernel<1>, grid_for(words), kThreads, 0, stream_, tables_,
+                           params.log_n, limbs, prime_base, polys, x, x_stride, d, y, y_stride);
+          return cudaGetLastError();
+        }),
+        "pointwise");
+}
+
+void Engine::encrypt_finish(int polys, int limbs, int prime_base, bool subtract, const int64_t *errors,
+                            const int64_t *plain, int64_t *ct) {
+  note_launch();
+  launch_chained(encrypt_finish_kernel, grid_for((static_cast<long long>(limbs) << params.log_n) * polys),
+                 kThreads, 0, stream_, tables_, params.log_n, limbs, prime_base, polys, subtract, errors, plain,
+                 ct);
+  check(cudaGetLastError(), "encrypt");
 }
 
 void Engine::tile(const int64_t *chain, int limbs, int prime_base, int64_t *y, long long y_stride) {
@@ -545,55 +638,34 @@ std::unique_ptr<Data> Engine::encrypt(const Data &pt, const Data &key) {
   const int n = params.n;
   const long long ps = static_cast<long long>(L) * n;
   auto ct = make_data(kUnitCiphertext, pt.flag & ~kFlagSpecial, mid, 2, pt.scale);
-  int64_t *c0 = ct->d, *c1 = ct->d + ps;
-  int64_t *chain = alloc_words(n);
-  if (key.type == kPublicKey) {
-    // CKKSCore::encrypt(pt, pk) (core.cpp:35-85).
-    if (key.moduli_id > mid)
-      throw std::runtime_error("Encrypt: the level of the input plaintext is greater than that of "
-                               "the input public key.");
-    int64_t *e0 = alloc_words(static_cast<size_t>(ps));
-    int64_t *e1 = alloc_words(static_cast<size_t>(ps));
-    int64_t *u = alloc_words(static_cast<size_t>(ps));
-    draw_gaussian(chain);
-    tile(chain, L, mid, e0, n);
-    draw_gaussian(chain);
-    tile(chain, L, mid, e1, n);
-    draw_uniform(chain, 0, 1, 0, 2, 0);
-    pointwise(kOpAddReduce, L, mid, pt.d, e0, nullptr, e0);
-    tile(chain, L, mid, u, n);
-    ntt_in_place(u, L, mid, ps, 1);
-    const long long off = static_cast<long long>(mid - key.moduli_id) * n;
-    const long long kps = key.poly_stride();
-    pointwise(kOpMult, L, mid, u, key.d + off, nullptr, c0);
-    pointwise(kOpMult, L, mid, u, key.d + kps + off, nullptr, c1);
-    intt_in_place(ct->d, L, mid, ps, 2);
-    pointwise(kOpAddReduce, L, mid, c0, e0, nullptr, c0);
-    pointwise(kOpAddReduce, L, mid, c1, e1, nullptr, c1);
-    free_words(e0);
-    free_words(e1);
-    free_words(u);
-  } else if (key.type == kSecretKey) {
-    // CKKSCore::encrypt(pt, sk) (core.cpp:87-122).
-    if (key.moduli_id > mid)
-      throw std::runtime_error("Encrypt: the level of the input plaintext is greater than that of "
-                               "the input secret key.");
-    int64_t *e = alloc_words(static_cast<size_t>(ps));
-    draw_gaussian(chain);
-    tile(chain, L, mid, e, n);
-    pointwise(kOpAddReduce, L, mid, pt.d, e, nullptr, e);
-    draw_uniform(c1, n, L, mid, 0, 0);
-    const int64_t *s = key.d + static_cast<long long>(mid - key.moduli_id) * n;
-    pointwise(kOpMult, L, mid, c1, s, nullptr, c0);
-    pointwise(kOpReduce, L, mid, c0, nullptr, nullptr, c0);
-    intt_in_place(ct->d, L, mid, ps, 2);
-    pointwise(kOpSubReduce, L, mid, e, c0, nullptr, c0);
-    free_words(e);
-  } else {
-    free_words(chain);
+  if (key.type != kPublicKey && key.type != kSecretKey)
     throw std::invalid_argument("Encrypt: the key is neither a public key nor a secret key.");
+  if (key.moduli_id > mid)
+    throw std::runtime_error(std::string("Encrypt: the level of the input plaintext is greater than that of "
+                                         "the input ") +
+                             (key.type == kPublicKey ? "public key." : "secret key."));
+  const long long off = static_cast<long long>(mid - key.moduli_id) * n;
+  int64_t *chains = alloc_words(3 * static_cast<size_t>(n));  // sampled polynomials
+  if (key.type == kPublicKey) {
+    // CKKSCore::encrypt(pt, pk) (core.cpp:35-85): two errors and the ternary polynomial.
+    int64_t *u = alloc_words(static_cast<size_t>(ps));
+    draw_gaussian(chains, 2, 1);
+    tile(chains + 2 * n, L, mid, u, n);
+    ntt_in_place(u, L, mid, ps, 1);
+    multiply_polys(2, L, mid, key.d + off, key.poly_stride(), u, ct->d, ps);
+    intt_in_place(ct->d, L, mid, ps, 2);
+    encrypt_finish(2, L, mid, false, chains, pt.d, ct->d);
+    free_words(u);
+  } else {
+    // CKKSCore::encrypt(pt, sk) (core.cpp:87-122).
+    int64_t *c0 = ct->d, *c1 = ct->d + ps;
+    draw_gaussian(chains);
+    draw_uniform(c1, n, L, mid, 0, 0);
+    pointwise(kOpMultReduce, L, mid, c1, key.d + off, nullptr, c0);
+    intt_in_place(ct->d, L, mid, ps, 2);
+    encrypt_finish(1, L, mid, true, chains, pt.d, ct->d);
   }
-  free_words(chain);
+  free_words(chains);
   return ct;
 }
 
