@@ -285,8 +285,8 @@ std::unique_ptr<Data> Engine::multiply_plain(const Data &ct, const Data &pt) {
   if (ct.level() <= 0 || pt.level() <= 0)
     throw std::runtime_error(fn + ": the input texts should have a positive level.");
   const int level = std::min(ct.level(), pt.level());
-  auto c = prepare_for_multiply(ct, level);
-  auto p = prepare_for_multiply(pt, level);
+  const auto prepared = prepare_pair(ct, pt, level);
+  const Data *c = prepared.first.get(), *p = prepared.second.get();
   auto out = make_data(kUnitCiphertext, (c->flag | p->flag) & ~kFlagRescaled, c->moduli_id,
                        c->polys, c->scale * p->scale);
   multiply_polys(c->polys, c->chains, c->moduli_id, c->d, c->poly_stride(), p->d, out->d, out->poly_stride());

@@ -39,7 +39,7 @@ const char *Data::type_name() const {
 
 Data::~Data() {
   if (engine) {
-    if (d) engine->release(d, copy_pending);
+    if (d && owns) engine->release(d, copy_pending);
     engine->forget(this);
   }
 }
@@ -235,7 +235,7 @@ Engine::~Engine() {
   // Objects still alive lose their device memory and their engine; the C ABI
   // rejects any later use of them.
   for (Data *d : live_) {
-    if (d->d) cudaFreeAsync(d->d, stream_);
+    if (d->d && d->owns) cudaFreeAsync(d->d, stream_);
     d->d = nullptr;
     d->engine = nullptr;
   }
@@ -606,7 +606,7 @@ std::unique_ptr<Data> Engine::rescale_to_ntt(const Data &ct, const ExactLimbs &e
   check(timed("rescale_to_ntt", [&] {
           return launch_rescale_to_ntt(tables_, ks_, params.log_n, ct.polys, out->chains,
                                        ct.moduli_id, ct.d, ct.poly_stride(), out->d,
-                                       out->poly_stride(), stream_, exact);
+                                       out->poly_stride(), stream_, exact, ct.polys, nullptr);
         }),
         "rescale to NTT");
   return out;
@@ -663,6 +663,40 @@ std::unique_ptr<Data> Engine::prepare_for_multiply(const Data &text, int level, 
   return cur;
 }
 
+std::pair<std::unique_ptr<Data>, std::unique_ptr<Data>> Engine::prepare_pair(const Data &a, const Data &b,
+                                                                             int level, const Data *rk) {
+  // Two coefficient-form texts at the level itself are rescaled and transformed in one
+  // launch a pass: one text of few limbs does not fill the machine.
+  const bool joint = a.level() == level && b.level() == level && a.moduli_id == b.moduli_id &&
+                     a.chains == b.chains && a.chains >= 2 && !a.is_rescaled() && !b.is_rescaled() &&
+                     !a.is_ntt() && !b.is_ntt() && (!rk || (a.polys == 2 && b.polys == 2));
+  if (!joint) return {prepare_for_multiply(a, level, rk), prepare_for_multiply(b, level, rk)};
+  const int mid = a.moduli_id;
+  ExactLimbs exact = rk ? relinearize_exact_limbs(mid + 1, *rk, 1) : ExactLimbs{ExactLimbs::kAllExact, 0};
+  exact.pairs = true;
+  auto pa = make_data(a.type, a.flag | kFlagRescaled | kFlagNtt, mid + 1, a.polys + b.polys,
+                      params.rescaled_scale(a.scale, mid));
+  auto pb = std::make_unique<Data>();  // the second half of pa's words
+  pb->engine = this;
+  pb->serial = ++serial_;
+  pb->type = b.type;
+  pb->flag = b.flag | kFlagRescaled | kFlagNtt;
+  pb->moduli_id = pa->moduli_id;
+  pb->polys = b.polys;
+  pb->chains = pa->chains;
+  pb->scale = params.rescaled_scale(b.scale, mid);
+  pb->owns = false;
+  pb->d = pa->d + a.polys * pa->poly_stride();
+  pa->polys = a.polys;
+  check(timed("rescale_to_ntt", [&] {
+          return launch_rescale_to_ntt(tables_, ks_, params.log_n, a.polys + b.polys, pa->chains, mid, a.d,
+                                       a.poly_stride(), pa->d, pa->poly_stride(), stream_, exact, a.polys,
+                                       b.d);
+        }),
+        "rescale to NTT");
+  return {std::move(pa), std::move(pb)};
+}
+
 void Engine::require_key_level(const std::string &fn, const Data &text, const Data &key,
                                bool for_multiply, const char *key_name) {
   // is_key_compatible (engine_require.cpp:24-32) with the multiply relaxation
@@ -692,8 +726,8 @@ std::unique_ptr<Data> Engine::multiply(const Data &a, const Data &b) {
   require_text(fn, a, 0, 2, 2, true);
   require_text(fn, b, 1, 2, 2, true);
   const int level = std::min(a.level(), b.level());
-  auto pa = prepare_for_multiply(a, level);
-  auto pb = prepare_for_multiply(b, level);
+  const auto prepared = prepare_pair(a, b, level);
+  const Data *pa = prepared.first.get(), *pb = prepared.second.get();
   const int flag = (pa->flag | pb->flag) & ~kFlagRescaled;
   auto out = make_data(kUnitCiphertext, flag, pa->moduli_id, 3, pa->scale * pb->scale);
   check(timed("tensor", [&] { return launch_tensor(tables_, params.n, pa->chains, pa->moduli_id, pa->d, pb->d, out->d, stream_); }),
@@ -859,8 +893,7 @@ std::unique_ptr<Data> Engine::multiply_relinearize(const Data &a, const Data &b,
   require_key_level(fn, a, rk, true);
   require_key_level(fn, b, rk, true);
   const int level = std::min(a.level(), b.level());
-  auto pa = prepare_for_multiply(a, level, &rk);
-  auto pb = prepare_for_multiply(b, level, &rk);
+  const auto [pa, pb] = prepare_pair(a, b, level, &rk);
   return relinearized_product(*pa, *pb, rk);
 }
 
@@ -945,8 +978,8 @@ std::unique_ptr<Data> Engine::multiply_relinearize_rescale(const Data &a, const 
   require_key_level(fn, a, rk, true);
   require_key_level(fn, b, rk, true);
   const int level = std::min(a.level(), b.level());
-  auto pa = prepare_for_multiply(a, level, &rk);
-  auto pb = prepare_for_multiply(b, level, &rk);
+  const auto prepared = prepare_pair(a, b, level, &rk);
+  const Data *pa = prepared.first.get(), *pb = prepared.second.get();
   const int m = pa->moduli_id;
   const int L = pa->chains;
   {

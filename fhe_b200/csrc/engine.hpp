@@ -106,6 +106,7 @@ struct Data {
   int64_t *d = nullptr;
   uint64_t serial = 0;  // unique per engine, never reused (keys captured graphs)
   mutable bool copy_pending = false;  // a download may still read d
+  bool owns = true;  // false: d lies inside another object, which outlives this one
 
   size_t words() const;
   long long poly_stride() const;
@@ -593,6 +594,9 @@ class Engine {
   // to_ntt(core_rescale(text)); limbs outside `exact` value-only.
   std::unique_ptr<Data> rescale_to_ntt(const Data &text,
                                        const ExactLimbs &exact = ExactLimbs{ExactLimbs::kAllExact, 0});
+  // prepare_for_multiply of both factors of a product.
+  std::pair<std::unique_ptr<Data>, std::unique_ptr<Data>> prepare_pair(const Data &a, const Data &b, int level,
+                                                                       const Data *rk = nullptr);
   std::unique_ptr<Data> relinearized_product(const Data &pa, const Data &pb, const Data &rk);
   // The limbs of polynomial `poly` of a product at moduli_id that relinearization
   // with rk reads word for word (ExactLimbs), or every limb exact when the switch is

@@ -22,9 +22,10 @@ namespace fhe_b200 {
 struct ExactLimbs {
   int poly = -1;      // -1: none; kAllExact: every limb of every polynomial
   uint64_t mask = 0;  // limbs below 64
+  bool pairs = false;  // the launch holds two texts of two polynomials: `poly` counts in each
   static constexpr int kAllExact = -2;
   __host__ __device__ bool exact(int p, int limb) const {
-    return poly == kAllExact || (p == poly && limb < 64 && ((mask >> limb) & 1) != 0);
+    return poly == kAllExact || ((pairs ? p & 1 : p) == poly && limb < 64 && ((mask >> limb) & 1) != 0);
   }
 };
 
@@ -409,13 +410,13 @@ cudaError_t launch_to_ntt(const PrimeTables &t, int log_n, int polys, int limbs,
                           cudaStream_t s);
 // to_ntt_ of the rescale of a coefficient-form text in one pass: x is [polys][limbs +
 // 1][N] at src_moduli_id, y is [polys][limbs][N] at src_moduli_id + 1 (NTT form).
-// Limbs outside `exact` (all of them exact by default) are transformed value-only: a
-// word of the same value modulo q, in [0, 2q).
+// Limbs outside `exact` are transformed value-only: a word of the same value modulo q, in
+// [0, 2q).  Polynomials from first_polys on are those of a second text of the same limbs.
 cudaError_t launch_rescale_to_ntt(const PrimeTables &t, const KeySwitchTables &ks, int log_n,
                                   int polys, int limbs, int src_moduli_id, const int64_t *x,
                                   long long x_stride, int64_t *y, long long y_stride,
-                                  cudaStream_t s,
-                                  const ExactLimbs &exact = ExactLimbs{ExactLimbs::kAllExact, 0});
+                                  cudaStream_t s, const ExactLimbs &exact, int first_polys,
+                                  const int64_t *second);
 // attach_special_prime_chains_ of a coefficient-form text: y [polys][limbs + K][N]
 // = to_ntt_ of (x * P on the limbs, zero special limbs); the zero limbs are written
 // as zeros (their transform), the others go through one fused NTT.

@@ -211,6 +211,8 @@ struct RescaleEnterLoad {
   };
   const int64_t *src;             // [poly][limbs + 1][N]
   long long poly_stride;
+  int first_polys;                // polynomials from this one on come from `second`
+  const int64_t *second;
   int dropped;                    // the dropped prime
   const int64_t *rescale_scale;   // its row, indexed by prime
   const int64_t *rescale_shoup;   // the same row's (C, C') pairs
@@ -221,7 +223,7 @@ struct RescaleEnterLoad {
   const int64_t *enter_shoup;  // the row's rescale_enter_shoup pairs
   ExactLimbs exact;            // MIXED
   __device__ __forceinline__ Raw raw(int poly, int limb, int gi, int n) const {
-    const int64_t *s = src + poly * poly_stride;
+    const int64_t *s = poly < first_polys ? src + poly * poly_stride : second + (poly - first_polys) * poly_stride;
     return {s[gi], s[static_cast<long long>(limb + 1) * n + gi]};
   }
   __device__ __forceinline__ int64_t word(Raw x, int poly, int limb, int prime) const {
