@@ -62,34 +62,46 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   const int P = ks.prime_count;
   const int64_t *x = acc + static_cast<long long>(poly) * (L + K) * n + coeff0;
 
-  // 1. Divisor triangle of one coefficient per thread, then its A row.
-  if (tid < kTcCoeffs) {
-    int64_t sp[K];
+  // 1. Divisor triangle, two adjacent lanes a coefficient: lane `side` holds the special
+  // limbs i = 2 j + side, and each step's divisor comes from its owner by a shuffle.  One
+  // thread a coefficient left half the warps waiting at the barrier below and ran a chain
+  // twice as long.  The lanes then write alternate 16-byte chunks of the A row.
+  {
+    const int c = tid >> 1, side = tid & 1;
+    constexpr int kOwn = (K + 1) / 2;
+    int64_t sp[kOwn];
 #pragma unroll
-    for (int i = 0; i < K; i++) sp[i] = x[static_cast<long long>(L + i) * n + tid];
+    for (int j = 0; j < kOwn; j++) {
+      const int i = 2 * j + side;
+      sp[j] = i < K ? x[static_cast<long long>(L + i) * n + c] : 0;
+    }
     uint64_t w[KB / 8];
 #pragma unroll
     for (int i = 0; i < KB / 8; i++) w[i] = 0;
 #pragma unroll
     for (int s = 0; s < K; s++) {
-      const int64_t d = sp[K - 1 - s];
+      const int64_t d = __shfl_sync(0xffffffffu, sp[(K - 1 - s) >> 1], (lane & ~1) | ((K - 1 - s) & 1));
       w[s] = static_cast<uint64_t>(d);
       if (d < 0) w[K + (s >> 3)] |= 1ull << (8 * (s & 7));
 #pragma unroll
-      for (int i = 0; i < K - 1 - s; i++) {
-        const int prime = moduli_id + L + i;
+      for (int j = 0; j < kOwn; j++) {
+        if (2 * j >= K - 1 - s) continue;
+        const int i = 2 * j + side;
+        // The odd lane has nothing left where the even one has its last product.
+        const int prime = moduli_id + L + (i < K - 1 - s ? i : i - 1);
         const uint64_t q = t.q[prime];
         const int64_t q2 = static_cast<int64_t>(q << 1);
-        sp[i] = mont_mult(guard(sp[i] + q2 - d, q2), ks.p_inverse_mult_r[s * P + prime], q,
-                          t.k[prime]);
+        const int64_t v = mont_mult(guard(sp[j] + q2 - d, q2), ks.p_inverse_mult_r[s * P + prime], q, t.k[prime]);
+        sp[j] = i < K - 1 - s ? v : sp[j];
       }
     }
 #pragma unroll
     for (int ch = 0; ch < KB / 16; ch++) {
+      if ((ch & 1) != side) continue;
       const uint4 v = make_uint4(static_cast<uint32_t>(w[2 * ch]), static_cast<uint32_t>(w[2 * ch] >> 32),
                                  static_cast<uint32_t>(w[2 * ch + 1]),
                                  static_cast<uint32_t>(w[2 * ch + 1] >> 32));
-      *reinterpret_cast<uint4 *>(sA + core_offset(tid, ch * 16, kTcCoeffs)) = v;
+      *reinterpret_cast<uint4 *>(sA + core_offset(c, ch * 16, kTcCoeffs)) = v;
     }
   }
   if (warp == 0) tmem_alloc(&tmem_base);
