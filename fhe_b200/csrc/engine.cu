@@ -498,12 +498,14 @@ const DevicePartitions &Engine::partitions(int moduli_id, int key_moduli_id) {
   // One device block: ints first, then the int64 tables.
   const size_t n_int = 3 * static_cast<size_t>(count);
   const size_t int_words = (n_int * sizeof(int) + 7) / 8;
-  const size_t words = int_words + static_cast<size_t>(count) * (16 + 256 + 16 * static_cast<size_t>(E));
+  const size_t words = int_words + static_cast<size_t>(count) * (2 * (16 + 256) + 16 * static_cast<size_t>(E));
   std::vector<int64_t> host(words, 0);
   int *ints = reinterpret_cast<int *>(host.data());
   int64_t *inv = host.data() + int_words;
   int64_t *prod = inv + static_cast<size_t>(count) * 16;
   int64_t *prod2 = prod + static_cast<size_t>(count) * 256;
+  int64_t *inv_plain = prod2 + static_cast<size_t>(count) * 16 * E;
+  int64_t *prod_plain = inv_plain + static_cast<size_t>(count) * 16;
   for (int p = 0; p < count; p++) {
     const auto &pt = parts[p];
     if (pt.size > 16) throw std::invalid_argument("partition larger than 16 limbs.");
@@ -517,10 +519,23 @@ const DevicePartitions &Engine::partitions(int moduli_id, int key_moduli_id) {
     dp.max_size = std::max(dp.max_size, pt.size);
     dp.size_mask |= 1u << pt.size;
     const auto pc = params.partition_constants(moduli_id, pt);
-    for (size_t i = 0; i < pc.inverse_r.size(); i++) inv[p * 16 + i] = pc.inverse_r[i];
+    // The plain residue (times R^-1) as the bits of a double.
+    auto plain = [&](int64_t mont, int limb) {
+      const int prime = moduli_id + pt.start + limb;
+      const uint64_t qi = params.q[prime];
+      const int64_t w = guard(mont_exit(guard(mont, static_cast<int64_t>(qi)), qi, params.k[prime]),
+                              static_cast<int64_t>(qi));
+      return static_cast<int64_t>(fp_raw(static_cast<double>(w)));
+    };
+    for (size_t i = 0; i < pc.inverse_r.size(); i++) {
+      inv[p * 16 + i] = pc.inverse_r[i];
+      inv_plain[p * 16 + i] = plain(pc.inverse_r[i], static_cast<int>(i) + 1);
+    }
     for (size_t ci = 0; ci < pc.product_r.size(); ci++)
-      for (size_t t2 = 0; t2 < pc.product_r[ci].size(); t2++)
+      for (size_t t2 = 0; t2 < pc.product_r[ci].size(); t2++) {
         prod[(p * 16 + ci) * 16 + t2] = pc.product_r[ci][t2];
+        prod_plain[(p * 16 + ci) * 16 + t2] = plain(pc.product_r[ci][t2], static_cast<int>(ci + t2) + 2);
+      }
     for (int ci = 0; ci + 1 < pt.size; ci++)
       for (int j = 0; j < E; j++)
         prod2[(static_cast<size_t>(p) * 16 + ci) * E + j] = pc.product_r_squared[static_cast<size_t>(ci) * E + j];
@@ -536,6 +551,8 @@ const DevicePartitions &Engine::partitions(int moduli_id, int key_moduli_id) {
   dp.inverse_r = d64;
   dp.product_r = d64 + static_cast<size_t>(count) * 16;
   dp.product_r_squared = dp.product_r + static_cast<size_t>(count) * 256;
+  dp.inverse_plain = reinterpret_cast<const double *>(dp.product_r_squared + static_cast<size_t>(count) * 16 * E);
+  dp.product_plain = dp.inverse_plain + static_cast<size_t>(count) * 16;
   return partition_cache_.emplace(key, dp).first->second;
 }
 

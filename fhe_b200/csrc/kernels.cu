@@ -152,6 +152,61 @@ __global__ void scalar_rescale_kernel(PrimeTables t, KeySwitchTables ks, int log
 
 // ---------------------------------------------------------- mixed radix --
 
+// Garner's digits of a partition whose limbs all have primes that fp_prime accepts, but
+// perhaps the last: the digits after the first are canonical residues (each is reduced to
+// [0, q) from a value in the lazy range), so any exact evaluation gives them.  Here a digit
+// is (x_j - Y_j) inverse_j in doubles (modarith.cuh), Y_j = x_0 + sum_i y_i product_ij kept
+// unreduced: a term is within 3/4 q of zero, so |Y_j| stays below 9 q and x_j - Y_j below
+// 2^45.  A last limb of another prime takes its Y as integers.  False where a word is
+// outside [0, 2q_j) or the first one outside [0, 2 q_j] for some j: the reference's steps are
+// then not canonical, and the caller takes them as written.
+template <int A>
+__device__ __forceinline__ bool garner_fp(const PrimeTables &t, const DevicePartitions &dp, int p, int prime0,
+                                          const int64_t (&xw)[A], int64_t (&y)[A]) {
+  const double *inverse = dp.inverse_plain + p * 16;
+  const double *product = dp.product_plain + p * 256;
+  bool ok = fp_prime(t.q[prime0]) && static_cast<uint64_t>(xw[0]) < 2 * t.q[prime0];
+#pragma unroll
+  for (int j = 1; j < A; j++) {
+    const uint64_t q2 = 2 * t.q[prime0 + j];
+    ok = ok && static_cast<uint64_t>(xw[j]) < q2 && static_cast<uint64_t>(xw[0]) <= q2;
+    if (j < A - 1) ok = ok && fp_prime(t.q[prime0 + j]);
+  }
+  if (!ok) return false;
+  const double first = fp_from_word(static_cast<uint64_t>(xw[0]));
+  const bool last_fp = fp_prime(t.q[prime0 + A - 1]);
+  double yd[A];
+#pragma unroll
+  for (int j = 0; j < A; j++) yd[j] = first;
+  y[0] = xw[0];
+  int64_t last = xw[0];
+  const uint64_t ql = t.q[prime0 + A - 1], kl = t.k[prime0 + A - 1];
+  const int64_t qls = static_cast<int64_t>(ql), ql2 = qls << 1;
+#pragma unroll
+  for (int ci = 0; ci < A - 1; ci++) {
+    const int yo = ci + 1;
+    if (yo == A - 1 && !last_fp) {
+      y[yo] = guard(mont_mult(guard(xw[yo] + ql2 - last, ql2), dp.inverse_r[p * 16 + ci], ql, kl), qls);
+      break;
+    }
+    const FpPrime f{fp_from_word(t.q[prime0 + yo]), t.inv_q[prime0 + yo]};
+    const double d = fp_canonical(
+        fp_mul(fp_from_word(static_cast<uint64_t>(xw[yo])) - yd[yo], inverse[ci], f), f);
+    y[yo] = fp_to_word(d);
+#pragma unroll
+    for (int t2 = 0; t2 < A - ci - 2; t2++) {
+      const int dst = yo + 1 + t2;
+      if (dst < A - 1 || last_fp) {
+        const FpPrime g{fp_from_word(t.q[prime0 + dst]), t.inv_q[prime0 + dst]};
+        yd[dst] += fp_mul(d, product[ci * 16 + t2], g);
+      } else {  // mont_enter_add_reduce_2q_to_q (compound.cpp:17-24)
+        last = guard(guard(mont_mult(y[yo], dp.product_r[(p * 16 + ci) * 16 + t2], ql, kl) + last, ql2), qls);
+      }
+    }
+  }
+  return true;
+}
+
 // One partition of alpha = A limbs per thread-coefficient (rns_to_mrs,
 // core_key_switch.cpp:21-56, Garner's algorithm with the reference's lazy ranges).
 // Three CTAs per SM where the digits fit the registers that leaves (A <= 10).
@@ -165,28 +220,30 @@ __global__ void __launch_bounds__(256, A <= 10 ? 3 : 2)
   const int start = dp.start[p];
   const int coeff = blockIdx.x * blockDim.x + threadIdx.x;
   if (coeff >= n) return;
-  int64_t y[A];
-  const int64_t first = x[static_cast<long long>(start) * n + coeff];
+  int64_t xw[A], y[A];
 #pragma unroll
-  for (int c = 0; c < A; c++) y[c] = first;
+  for (int c = 0; c < A; c++) xw[c] = x[static_cast<long long>(start + c) * n + coeff];
+  if (A == 1 || dp.inverse_plain == nullptr || !garner_fp<A>(t, dp, p, moduli_id + start, xw, y)) {
 #pragma unroll
-  for (int ci = 0; ci < A - 1; ci++) {
-    const int yo = ci + 1;
-    const int prime = moduli_id + start + yo;
-    const uint64_t q = t.q[prime], k = t.k[prime];
-    const int64_t qs = static_cast<int64_t>(q), q2 = qs << 1;
-    const int64_t xv = x[static_cast<long long>(start + yo) * n + coeff];
-    // mont_sub_enter_reduce_2q_to_q (compound.cpp:36-43)
-    y[yo] = guard(mont_mult(guard(xv + q2 - y[yo], q2), dp.inverse_r[p * 16 + ci], q, k), qs);
+    for (int c = 0; c < A; c++) y[c] = xw[0];
 #pragma unroll
-    for (int t2 = 0; t2 < A - ci - 2; t2++) {
-      const int dst = yo + 1 + t2;
-      const int prime2 = moduli_id + start + dst;
-      const uint64_t qq = t.q[prime2], kk = t.k[prime2];
-      const int64_t qqs = static_cast<int64_t>(qq), qq2 = qqs << 1;
-      // mont_enter_add_reduce_2q_to_q (compound.cpp:17-24)
-      y[dst] = guard(guard(mont_mult(y[yo], dp.product_r[(p * 16 + ci) * 16 + t2], qq, kk) + y[dst],
-                           qq2), qqs);
+    for (int ci = 0; ci < A - 1; ci++) {
+      const int yo = ci + 1;
+      const int prime = moduli_id + start + yo;
+      const uint64_t q = t.q[prime], k = t.k[prime];
+      const int64_t qs = static_cast<int64_t>(q), q2 = qs << 1;
+      // mont_sub_enter_reduce_2q_to_q (compound.cpp:36-43)
+      y[yo] = guard(mont_mult(guard(xw[yo] + q2 - y[yo], q2), dp.inverse_r[p * 16 + ci], q, k), qs);
+#pragma unroll
+      for (int t2 = 0; t2 < A - ci - 2; t2++) {
+        const int dst = yo + 1 + t2;
+        const int prime2 = moduli_id + start + dst;
+        const uint64_t qq = t.q[prime2], kk = t.k[prime2];
+        const int64_t qqs = static_cast<int64_t>(qq), qq2 = qqs << 1;
+        // mont_enter_add_reduce_2q_to_q (compound.cpp:17-24)
+        y[dst] = guard(guard(mont_mult(y[yo], dp.product_r[(p * 16 + ci) * 16 + t2], qq, kk) + y[dst],
+                             qq2), qqs);
+      }
     }
   }
 #pragma unroll

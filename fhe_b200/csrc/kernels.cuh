@@ -43,6 +43,10 @@ struct DevicePartitions {
   int key_index_first[8] = {};        // host copy of key_index[0 .. 7]
   int64_t *inverse_r = nullptr;       // [count][16]
   int64_t *product_r = nullptr;       // [count][16][16]
+  // The plain residues of both as doubles for fp_prime limbs; null where only the words
+  // above were made (fhe_relinearize_noalloc).
+  const double *inverse_plain = nullptr;  // [count][16]
+  const double *product_plain = nullptr;  // [count][16][16]
   int64_t *product_r_squared = nullptr;  // [count][16][extended]
 };
 
