@@ -1,5 +1,4 @@
-// The output stage of a ModDown epilogue, shared by the CUDA-core and the
-// tensor-core kernels: the divided limbs (the exact division by the special primes,
+// The output stage of the CUDA-core ModDown epilogue: the divided limbs (the exact division by the special primes,
 // make_unsigned_reduce_2q_to_q, canonical in [0, q)) combined with the caller's
 // operations (core_key_switch.cpp:110-160 and its callers).
 #pragma once
@@ -12,9 +11,8 @@ namespace fhe_b200 {
 // A CTA owns coefficients [coeff0, coeff0 + valid) of polynomial `poly`; divide(j, c)
 // gives the divided limb j of coefficient coeff0 + c.  first_limb holds at least
 // `valid` words of shared memory.  Every thread of the CTA calls this.  The rescale's
-// product is Shoup's when its operand is in range (rescale_word_shoup, same word);
-// LAZY is kept for the callers' signatures and selects nothing else.
-template <bool LAZY = false, class Divide>
+// product is Shoup's when its operand is in range (rescale_word_shoup, same word).
+template <class Divide>
 __device__ __forceinline__ void mod_down_store(const PrimeTables &t, const KeySwitchTables &ks,
                                                int n, int moduli_id, int L, int poly, int coeff0,
                                                int valid, const EpilogueOps &ops, int64_t *out,

@@ -209,9 +209,10 @@ __device__ __forceinline__ bool garner_fp(const PrimeTables &t, const DevicePart
 
 // One partition of alpha = A limbs per thread-coefficient (rns_to_mrs,
 // core_key_switch.cpp:21-56, Garner's algorithm with the reference's lazy ranges).
-// Three CTAs per SM where the digits fit the registers that leaves (A <= 10).
+// Six CTAs per SM where the digits fit the registers that leaves (A <= 10).
+constexpr int kMixedRadixThreads = 128;
 template <int A>
-__global__ void __launch_bounds__(256, A <= 10 ? 3 : 2)
+__global__ void __launch_bounds__(kMixedRadixThreads, A <= 10 ? 6 : 4)
     mixed_radix_kernel(PrimeTables t, DevicePartitions dp, int n, int moduli_id,
                                    const int64_t *x, int64_t *digits) {
   chained_kernel_begin();
@@ -606,13 +607,13 @@ cudaError_t launch_scalar_rescale(const PrimeTables &t, const KeySwitchTables &k
 
 cudaError_t launch_mixed_radix(const PrimeTables &t, const DevicePartitions &dp, int n,
                                int moduli_id, const int64_t *x, int64_t *digits, cudaStream_t s) {
-  const dim3 grid(blocks_for(n), dp.count);
+  const dim3 grid((n + kMixedRadixThreads - 1) / kMixedRadixThreads, dp.count);
   // One launch per distinct partition size; blocks of other sizes exit at once.
   for (int size = 1; size <= 16; size++) {
     if (!(dp.size_mask & (1u << size))) continue;
     switch (size) {
 #define FHE_MRS_CASE(A) \
-  case A: note_launch(); launch_chained(mixed_radix_kernel<A>, grid, kThreads, 0, s, t, dp, n, moduli_id, x, digits); break;
+  case A: note_launch(); launch_chained(mixed_radix_kernel<A>, grid, kMixedRadixThreads, 0, s, t, dp, n, moduli_id, x, digits); break;
       FHE_MRS_CASE(1) FHE_MRS_CASE(2) FHE_MRS_CASE(3) FHE_MRS_CASE(4) FHE_MRS_CASE(5)
       FHE_MRS_CASE(6) FHE_MRS_CASE(7) FHE_MRS_CASE(8) FHE_MRS_CASE(9) FHE_MRS_CASE(10)
       FHE_MRS_CASE(11) FHE_MRS_CASE(12) FHE_MRS_CASE(13) FHE_MRS_CASE(14) FHE_MRS_CASE(15)

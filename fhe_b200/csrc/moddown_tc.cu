@@ -20,14 +20,17 @@
 //     targets, so a CTA holds 128 tensor-memory columns and the B of one round, and
 //     four CTAs fit on an SM.
 // The epilogue folds the 8 partial sums into a 128-bit word, takes one REDC of it
-// (a word below q_j + 2^19), adds x_j prod pinv (one Montgomery product) and
-// reduces the total (below 4 q_j) to [0, q_j).
+// (a word below q_j + 2^19), adds x_j prod pinv (one Shoup product) and reduces the
+// total (below 4 q_j) to [0, q_j).  A target whose prime fp_prime accepts has plain
+// constants (no factor R) and is folded, added and rescaled in doubles: about 30
+// instructions in place of 90.  Each thread finishes its targets in registers (the rescale's
+// dropped limb, target 0, goes to the other half through shared memory first), and the
+// next round's B is copied while this one is folded, the first under the triangle.
 // The divisor triangle (K(K-1)/2 divisions per coefficient) stays on the CUDA
 // cores, as in the CUDA-core form.
 #include <cstring>
 #include <vector>
 
-#include "epilogue.cuh"
 #include "kernels.cuh"
 #include "modarith.cuh"
 #include "umma.cuh"
@@ -48,10 +51,10 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
                        TcStatus status) {
   chained_kernel_begin();
   constexpr int KB = row_bytes(K);
+  constexpr int kBBytes = kTcColumns * KB;
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t *sA = smem;                   // [128 rows][KB], core matrices
-  uint8_t *sB = smem + kTcCoeffs * KB;  // one round: [128 columns][KB]
-  int64_t *divided = reinterpret_cast<int64_t *>(sB + kTcColumns * KB);
+  uint8_t *sB = smem + kTcCoeffs * KB;  // two rounds: [128 columns][KB] each
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_base;
   __shared__ int64_t first_limb[kTcCoeffs];
@@ -62,17 +65,22 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   const int P = ks.prime_count;
   const int64_t *x = acc + static_cast<long long>(poly) * (L + K) * n + coeff0;
 
-  // 1. Divisor triangle, two adjacent lanes a coefficient: lane `side` holds the special
-  // limbs i = 2 j + side, and each step's divisor comes from its owner by a shuffle.  One
-  // thread a coefficient left half the warps waiting at the barrier below and ran a chain
-  // twice as long.  The lanes then write alternate 16-byte chunks of the A row.
-  {
-    const int c = tid >> 1, side = tid & 1;
-    constexpr int kOwn = (K + 1) / 2;
+  load_b_round<KB>(sB, tc.b, 0);
+
+  // 1. Divisor triangle.  From eight special primes on, two adjacent lanes share a
+  // coefficient: lane `side` holds the special limbs i = 2 j + side, and each step's divisor
+  // comes from its owner by a shuffle; one thread a coefficient left half the warps waiting
+  // at the barrier below and ran a chain twice as long (K = 10: serve_n16 10946 -> 10585 us;
+  // K = 4 with two lanes: eight hoisted rotations 1307 -> 1326 us).  The lanes then write
+  // alternate 16-byte chunks of the A row.
+  constexpr int kLanes = K >= 8 ? 2 : 1;
+  if (tid < kTcCoeffs * kLanes) {
+    const int c = tid / kLanes, side = tid % kLanes;
+    constexpr int kOwn = (K + kLanes - 1) / kLanes;
     int64_t sp[kOwn];
 #pragma unroll
     for (int j = 0; j < kOwn; j++) {
-      const int i = 2 * j + side;
+      const int i = kLanes * j + side;
       sp[j] = i < K ? x[static_cast<long long>(L + i) * n + c] : 0;
     }
     uint64_t w[KB / 8];
@@ -80,13 +88,15 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
     for (int i = 0; i < KB / 8; i++) w[i] = 0;
 #pragma unroll
     for (int s = 0; s < K; s++) {
-      const int64_t d = __shfl_sync(0xffffffffu, sp[(K - 1 - s) >> 1], (lane & ~1) | ((K - 1 - s) & 1));
+      const int own = (K - 1 - s) / kLanes;
+      const int64_t d = kLanes == 1 ? sp[own]
+                                    : __shfl_sync(0xffffffffu, sp[own], (lane & ~1) | ((K - 1 - s) & 1));
       w[s] = static_cast<uint64_t>(d);
       if (d < 0) w[K + (s >> 3)] |= 1ull << (8 * (s & 7));
 #pragma unroll
       for (int j = 0; j < kOwn; j++) {
-        if (2 * j >= K - 1 - s) continue;
-        const int i = 2 * j + side;
+        if (kLanes * j >= K - 1 - s) continue;
+        const int i = kLanes * j + side;
         // The odd lane has nothing left where the even one has its last product.
         const int prime = moduli_id + L + (i < K - 1 - s ? i : i - 1);
         const uint64_t q = t.q[prime];
@@ -97,7 +107,7 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
     }
 #pragma unroll
     for (int ch = 0; ch < KB / 16; ch++) {
-      if ((ch & 1) != side) continue;
+      if (ch % kLanes != side) continue;
       const uint4 v = make_uint4(static_cast<uint32_t>(w[2 * ch]), static_cast<uint32_t>(w[2 * ch] >> 32),
                                  static_cast<uint32_t>(w[2 * ch + 1]),
                                  static_cast<uint32_t>(w[2 * ch + 1] >> 32));
@@ -106,6 +116,7 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   }
   if (warp == 0) tmem_alloc(&tmem_base);
   if (tid == 0) mbar_init(&mbar);
+  async_copies_wait();
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -113,27 +124,97 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   const uint32_t tmem = tmem_base;
   const uint32_t bar = smem_addr(&mbar);
 
-  // 3. One MMA round per 16 targets; each thread folds 8 targets of its coefficient.
+  // 2. One MMA round per 16 targets; each thread finishes 8 targets of its coefficient.
   const int lane_base = (warp & 3) * 32;
   const int row = lane_base + lane;
   const int half = warp >> 2;
+  const uint32_t tmem_row = tmem + (static_cast<uint32_t>(lane_base) << 16);
+  const int64_t *base = poly < ops.base_polys  // uniform per CTA
+                            ? ops.base + static_cast<long long>(poly) * L * n + coeff0 + row
+                            : nullptr;
+  // Target j: x_j divided by the special primes, canonical, and the caller's addend.
+  auto divided = [&](int j, const uint32_t *d, int64_t xj) -> int64_t {
+    const int prime = moduli_id + j;
+    const uint64_t q = t.q[prime];
+    int64_t v;
+    if (fp_prime(q) && (static_cast<uint64_t>(xj) >> kFpWordBits) == 0) {
+      const FpPrime f{fp_from_word(q), t.inv_q[prime]};
+      const double sum = fold_fp(d, f) + fp_mul(fp_from_word(static_cast<uint64_t>(xj)),
+                                                fp_from_word(static_cast<uint64_t>(tc.c_shoup[2 * j])), f);
+      v = fp_to_word(fp_canonical(fp_reduce(sum, f), f));
+    } else {
+      uint64_t lo, hi;
+      fold8(d, lo, hi);
+      // REDC(X) < q + 2^19, and x_j prod pinv by Shoup's product is below 2q.  (A plain sum of
+      // an fp_prime target whose word is out of range takes one more factor R.)
+      if (fp_prime(q)) {
+        const uint64_t r = static_cast<uint64_t>(redc_wide(lo, hi, q, t.k[prime]));
+        lo = static_cast<uint64_t>(mont_mult(static_cast<int64_t>(r), t.r_squared[prime], q, t.k[prime]));
+      } else {
+        lo = static_cast<uint64_t>(redc_wide(lo, hi, q, t.k[prime]));
+      }
+      const uint64_t u = lo + shoup_mult(static_cast<uint64_t>(tc.c_shoup[2 * j]),
+                                         static_cast<uint64_t>(tc.c_shoup[2 * j + 1]),
+                                         static_cast<uint64_t>(xj), q);
+      uint64_t r = u >= (q << 1) ? u - (q << 1) : u;
+      v = static_cast<int64_t>(r >= q ? r - q : r);
+    }
+    if (base == nullptr) return v;
+    const int64_t qs = static_cast<int64_t>(q);
+    return guard(guard(base[static_cast<long long>(j) * n] + v, qs << 1), qs);
+  };
+  const int32_t place = ops.signed_perm == nullptr ? 0 : ops.signed_perm[coeff0 + row];
+  const uint64_t q_half = t.q[moduli_id] >> 1;  // of the dropped prime (unsigned, as get_rounder)
+  const long long rescale_row = static_cast<long long>(moduli_id) * P;
+  int64_t y0 = 0;
+  // Target j's word on its way out: rescaled by the first limb (core_rescale.cpp:5-25), moved
+  // by the caller's permutation (rotate_ after key_switch_mod_down, core.cpp:939-952), or as
+  // it is.
+  auto put = [&](int j, int64_t v) {
+    const int prime = moduli_id + j;
+    const uint64_t q = t.q[prime];
+    const int64_t qs = static_cast<int64_t>(q), q2 = qs << 1;
+    if (ops.rescale) {
+      if (j == 0) return;
+      const bool up = static_cast<uint64_t>(y0) > q_half;
+      const int64_t *shoup = ks.rescale_shoup + 2 * (rescale_row + prime);
+      if (fp_prime(q) && static_cast<uint64_t>(v) < static_cast<uint64_t>(q2) &&
+          static_cast<uint64_t>(y0) <= static_cast<uint64_t>(q2)) {
+        // Both words in the lazy range: the difference's product is canonical.
+        const FpPrime f{fp_from_word(q), t.inv_q[prime]};
+        double r = fp_canonical(fp_mul(fp_from_word(static_cast<uint64_t>(v)) - fp_from_word(static_cast<uint64_t>(y0)),
+                                       fp_from_word(static_cast<uint64_t>(shoup[0])), f), f);
+        r = up ? r + 1.0 : r;
+        v = fp_to_word(r >= f.q ? r - f.q : r);
+      } else {
+        v = rescale_word_shoup(v, y0, up ? 1 : 0, q, t.k[prime], ks.rescale_scale[rescale_row + prime], shoup);
+      }
+      out[static_cast<long long>(poly) * (L - 1) * n + static_cast<long long>(j - 1) * n + coeff0 + row] = v;
+      return;
+    }
+    int at = coeff0 + row;
+    if (ops.signed_perm != nullptr) {
+      if (place < 0) v = -v;
+      v = v < 0 ? v + qs : guard(v, qs);
+      at = place < 0 ? ~place : place;
+    }
+    out[static_cast<long long>(poly) * L * n + static_cast<long long>(j) * n + at] = v;
+  };
+
   bool ok = true;
   int round = 0;
   for (; round < tc.rounds; round++) {
-    {
-      // The round's slice of the constant B matrix, already in core-matrix order
-      // (the previous round's MMAs have completed: every thread passed its wait).
-      constexpr int chunks = kTcColumns * KB / 16;
-      const uint4 *src = reinterpret_cast<const uint4 *>(tc.b) + static_cast<size_t>(round) * chunks;
-      uint4 *dst = reinterpret_cast<uint4 *>(sB);
-      for (int i = tid; i < chunks; i += kTcThreads) dst[i] = src[i];
+    if (round > 0) {
+      async_copies_wait();
       fence_async_smem();
       __syncthreads();
     }
     if (tid == 0) {
-      mma_round(tmem, sA, sB, KB);
+      mma_round(tmem, sA, sB + (round & 1) * kBBytes, KB);
       mma_commit(bar);
     }
+    // The other buffer's MMAs have completed: every thread passed their wait.
+    if (round + 1 < tc.rounds) load_b_round<KB>(sB + ((round + 1) & 1) * kBBytes, tc.b, round + 1);
     // This thread's words x_j of the round, loaded while the MMAs run.
     constexpr int kHalfTargets = kTcTargets / 2;
     int64_t xs[kHalfTargets];
@@ -145,33 +226,25 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
     ok = __syncthreads_and(mbar_wait(bar, round & 1, status.wait_limit)) != 0;
     if (!ok) break;
     tc_fence_after();
-    // Each warpgroup folds 8 of the round's 16 targets, two per tensor-memory load.
+    if (round == 0 && ops.rescale) {
+      if (half == 0) {
+        uint32_t d[16];
+        tmem_load16(tmem_row, d);
+        first_limb[row] = divided(0, d, xs[0]);
+      }
+      __syncthreads();
+      y0 = first_limb[row];
+    }
 #pragma unroll
     for (int u2 = 0; u2 < kHalfTargets / 2; u2++) {
       const int jp = half * kHalfTargets + 2 * u2;
       const int j0 = round * kTcTargets + jp;
       if (j0 >= L) continue;  // uniform across the warp
       uint32_t d[16];
-      tmem_load16(tmem + (static_cast<uint32_t>(lane_base) << 16) + jp * 8, d);
+      tmem_load16(tmem_row + jp * 8, d);
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int j = j0 + h;
-        if (j >= L) continue;  // uniform across the warp
-        const int prime = moduli_id + j;
-        const uint64_t q = t.q[prime], kq = t.k[prime];
-        uint64_t lo, hi;
-        fold8(d + 8 * h, lo, hi);
-        const int64_t xj = xs[2 * u2 + h];
-        // REDC(X) < q + 2^19, and x_j prod pinv by Shoup's product is below 2q (its
-        // value is all that matters: the total is reduced to [0, q) below).
-        const uint64_t v = static_cast<uint64_t>(redc_wide(lo, hi, q, kq)) +
-                           shoup_mult(static_cast<uint64_t>(tc.c_shoup[2 * j]),
-                                      static_cast<uint64_t>(tc.c_shoup[2 * j + 1]),
-                                      static_cast<uint64_t>(xj), q);
-        uint64_t r = v >= (q << 1) ? v - (q << 1) : v;
-        r = r >= q ? r - q : r;
-        divided[j * kTcCoeffs + row] = static_cast<int64_t>(r);
-      }
+      for (int h = 0; h < 2; h++)
+        if (j0 + h < L) put(j0 + h, divided(j0 + h, d + 8 * h, xs[2 * u2 + h]));
     }
     tc_fence_before();
     __syncthreads();
@@ -180,6 +253,7 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   if (!ok) {
     // The round's MMAs may still be running: wait for them (bounded) before the
     // tensor memory is given back.
+    async_copies_wait();
     if (tid == 0) *static_cast<volatile int *>(status.error) = 1;
     if (warp == 0) mbar_wait(bar, round & 1);
   }
@@ -187,17 +261,10 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   __syncthreads();
   tc_fence_after();
   if (warp == 0) tmem_dealloc(tmem);
-  if (!ok) return;
-
-  // 4. The caller's operations on the divided limbs.
-  mod_down_store<true>(t, ks, n, moduli_id, L, poly, coeff0, kTcCoeffs, ops, out, first_limb,
-                       [&](int j, int c) -> int64_t { return divided[j * kTcCoeffs + c]; });
 }
 
-size_t tc_smem_bytes(int K, int L) {
-  const int kb = row_bytes(K);
-  return static_cast<size_t>(kTcCoeffs) * kb + static_cast<size_t>(kTcColumns) * kb +
-         static_cast<size_t>(L) * kTcCoeffs * sizeof(int64_t);
+size_t tc_smem_bytes(int K) {
+  return static_cast<size_t>(kTcCoeffs + 2 * kTcColumns) * row_bytes(K);
 }
 
 using u128 = unsigned __int128;
@@ -218,7 +285,7 @@ uint64_t pow_mod(uint64_t b, uint64_t e, uint64_t m) {
 
 bool mod_down_tc_supported(int special_count, int limbs, int n) {
   return special_count >= 1 && special_count <= 16 && limbs >= 1 && n >= kTcCoeffs &&
-         n % kTcCoeffs == 0 && tc_smem_bytes(special_count, limbs) <= 200 * 1024;
+         n % kTcCoeffs == 0;
 }
 
 ModDownTcHost make_mod_down_tc_tables(const std::vector<uint64_t> &q,
@@ -250,7 +317,8 @@ ModDownTcHost make_mod_down_tc_tables(const std::vector<uint64_t> &q,
     const int round = j / kTcTargets, jl = j % kTcTargets;
     uint8_t *b = h.b.data() + static_cast<size_t>(round) * kTcColumns * h.kb;
     for (int s = 0; s < K; s++) {
-      const uint64_t wn = mul_mod((m - w[s]) % m, r, m);  // w'_sj R
+      // w'_sj R, or plain where the target is folded in doubles
+      const uint64_t wn = fp_prime(m) ? (m - w[s]) % m : mul_mod((m - w[s]) % m, r, m);
       const uint64_t z = (m - mul_mod(two64, wn, m)) % m;  // -2^64 w'_sj R
       uint64_t e = wn;  // w'_sj 2^(8a) R for a = 0, 1, ...
       for (int a = 0; a < 8; a++) {
@@ -275,7 +343,7 @@ cudaError_t launch_mod_down_epilogue_tc(const PrimeTables &t, const KeySwitchTab
       (ops.base_polys > 0 && ops.base == nullptr) || (ops.rescale && ops.signed_perm != nullptr) ||
       ops.polys < 1 || ops.polys > 2 || ops.base_polys > ops.polys)
     return cudaErrorInvalidValue;
-  const size_t smem = tc_smem_bytes(K, limbs);
+  const size_t smem = tc_smem_bytes(K);
   const dim3 grid(n / kTcCoeffs, ops.polys);
   // The shared-memory limit is raised once per instantiation and device to the most
   // any supported shape needs, so no attribute call falls inside a graph capture.

@@ -13,7 +13,10 @@
 //     sums D_b = sum_(i,a) d_i[a] e_iaj[b] (each below 2^23) give
 //     X_j = sum_b D_b 2^(8b) = sum_(i,a) d_i[a] e_iaj == sum_i d_i C_ij (mod q_j),
 //     with X_j below 2^80;
-//   * one REDC of X_j on the CUDA cores leaves a word below q_j + 2^18 < 2 q_j.
+//   * one REDC of X_j on the CUDA cores leaves a word below q_j + 2^18 < 2 q_j; a target
+//     whose prime fp_prime accepts has constants C_ij R^-1 and is folded in doubles
+//     (fold_fp), about 25 instructions in place of 50.
+// The next round's B is copied while this one is folded.
 // A coefficient with a digit of 2^61 or more takes the reference's chain term by
 // term.  The values equal mod_up_contract_kernel's.
 #include "kernels.cuh"
@@ -38,8 +41,9 @@ __global__ void __launch_bounds__(kTcThreads, 4)
   if (dp.size[p] != A) return;  // uniform per CTA, before any barrier
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t *sA = smem;                                               // [128][KB]
-  uint8_t *sB = smem + kTcCoeffs * KB;                              // one round: [128][KB]
-  int64_t *sd = reinterpret_cast<int64_t *>(sB + kTcColumns * KB);  // [A][128] digits
+  uint8_t *sB = smem + kTcCoeffs * KB;                         // two rounds: [128][KB] each
+  constexpr int kBBytes = kTcColumns * KB;
+  int64_t *sd = reinterpret_cast<int64_t *>(sB + 2 * kBBytes);  // [A][128] digits
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_base;
   __shared__ int fast[kTcCoeffs];
@@ -48,6 +52,9 @@ __global__ void __launch_bounds__(kTcThreads, 4)
   const int coeff0 = blockIdx.x * kTcCoeffs;
   const int start = dp.start[p];
   const int E = dp.extended;
+
+  const uint8_t *bp = tc.b + tc.b_offset[p];
+  load_b_round<KB>(sB, bp, 0);
 
   // 1. Digits of one coefficient per thread: the A row, a copy for the quotients.
   if (tid < kTcCoeffs) {
@@ -73,6 +80,7 @@ __global__ void __launch_bounds__(kTcThreads, 4)
   }
   if (warp == 0) tmem_alloc(&tmem_base);
   if (tid == 0) mbar_init(&mbar);
+  async_copies_wait();
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
@@ -84,23 +92,21 @@ __global__ void __launch_bounds__(kTcThreads, 4)
   const int row = lane_base + lane;
   const int half = warp >> 2;
   const int64_t *cst = dp.product_r_squared + static_cast<long long>(p) * 16 * E;
-  const uint8_t *bp = tc.b + tc.b_offset[p];
   int64_t *out = ext + static_cast<long long>(p) * E * n + coeff0 + row;
   bool ok = true;
   int round = 0;
   for (; round < tc.rounds; round++) {
-    {
-      constexpr int chunks = kTcColumns * KB / 16;
-      const uint4 *src = reinterpret_cast<const uint4 *>(bp) + static_cast<size_t>(round) * chunks;
-      uint4 *dst = reinterpret_cast<uint4 *>(sB);
-      for (int i = tid; i < chunks; i += kTcThreads) dst[i] = src[i];
+    if (round > 0) {
+      async_copies_wait();
       fence_async_smem();
       __syncthreads();
     }
     if (tid == 0) {
-      mma_round(tmem, sA, sB, KB);
+      mma_round(tmem, sA, sB + (round & 1) * kBBytes, KB);
       mma_commit(bar);
     }
+    // The other buffer's MMAs have completed: every thread passed their wait.
+    if (round + 1 < tc.rounds) load_b_round<KB>(sB + ((round + 1) & 1) * kBBytes, bp, round + 1);
     ok = __syncthreads_and(mbar_wait(bar, round & 1, status.wait_limit)) != 0;
     if (!ok) break;
     tc_fence_after();
@@ -117,7 +123,10 @@ __global__ void __launch_bounds__(kTcThreads, 4)
         if (skip_own && j >= start && j < start + A) continue;  // uniform across the warp
         const int prime = moduli_id + j;
         const uint64_t q = t.q[prime], kq = t.k[prime];
-        if (fast[row]) {
+        if (fast[row] && fp_prime(q)) {
+          const FpPrime f{fp_from_word(q), t.inv_q[prime]};
+          out[static_cast<long long>(j) * n] = fp_to_word(fp_reduce(fold_fp(d + 8 * h, f), f) + f.q);
+        } else if (fast[row]) {
           uint64_t lo, hi;
           fold8(d + 8 * h, lo, hi);
           out[static_cast<long long>(j) * n] = redc_wide(lo, hi, q, kq);
@@ -137,6 +146,7 @@ __global__ void __launch_bounds__(kTcThreads, 4)
     tc_fence_after();
   }
   if (!ok) {
+    async_copies_wait();
     if (tid == 0) *static_cast<volatile int *>(status.error) = 1;
     if (warp == 0) mbar_wait(bar, round & 1);
   }
@@ -148,7 +158,7 @@ __global__ void __launch_bounds__(kTcThreads, 4)
 
 size_t mod_up_tc_smem(int A) {
   const int kb = digit_row_bytes(A);
-  return static_cast<size_t>(kTcCoeffs) * kb * 2 + static_cast<size_t>(A) * kTcCoeffs * 8;
+  return static_cast<size_t>(kTcCoeffs + 2 * kTcColumns) * kb + static_cast<size_t>(A) * kTcCoeffs * 8;
 }
 
 }  // namespace
@@ -179,7 +189,13 @@ ModUpTcHost make_mod_up_tc_tables(const std::vector<uint64_t> &q,
         const uint64_t c = i == 0 ? static_cast<uint64_t>(r_squared[moduli_id + j])
                                   : static_cast<uint64_t>(
                                         constants[p].product_r_squared[static_cast<size_t>(i - 1) * E + j]);
-        uint64_t e = c % qj;  // C_ij 2^(8a) mod q_j for a = 0, 1, ...
+        uint64_t e = c % qj;  // C_ij 2^(8a) mod q_j for a = 0, 1, ...; plain (R^-1) in doubles
+        if (fp_prime(qj)) {
+          u128 inv = 1, base = (u128(1) << 62) % qj;  // R^-1 = R^(q-2)
+          for (uint64_t x = qj - 2; x > 0; x >>= 1, base = base * base % qj)
+            if (x & 1) inv = inv * base % qj;
+          e = static_cast<uint64_t>(e * inv % qj);
+        }
         for (int a = 0; a < 8; a++) {
           for (int bb = 0; bb < 8; bb++)
             round[core_offset(jl * 8 + bb, i * 8 + a, kTcColumns)] = static_cast<uint8_t>(e >> (8 * bb));

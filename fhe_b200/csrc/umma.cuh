@@ -9,6 +9,8 @@
 
 #include <cuda_runtime.h>
 
+#include "modarith.cuh"
+
 namespace fhe_b200 {
 namespace umma {
 
@@ -126,6 +128,29 @@ __device__ __forceinline__ void mma_round(uint32_t tmem, const uint8_t *a, const
                                   (kTcColumns / 8) * 128, 128);
     mma_i8(tmem, da, db, kTcIdesc, k > 0 ? 1u : 0u);
   }
+}
+
+// 16-byte asynchronous copies to shared memory; async_copies_wait waits for this thread's.
+__device__ __forceinline__ void async_copy16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The B operand of round `round` (128 columns of kb bytes) on its way to shared memory.
+template <int KB>
+__device__ __forceinline__ void load_b_round(uint8_t *dst, const uint8_t *b, int round) {
+  constexpr int kChunks = kTcColumns * KB / 16;
+  const uint8_t *src = b + static_cast<size_t>(round) * kTcColumns * KB;
+  for (int i = threadIdx.x; i < kChunks; i += kTcThreads) async_copy16(dst + 16 * i, src + 16 * i);
+}
+
+// The same sum for a prime that fp_prime accepts (constants below 2^41: byte columns 6 and
+// 7 are zero), as a double congruent to it modulo q: hi 2^24 + lo with lo, hi < 2^41, the
+// product taken modulo q; within q / 2 + 2^41 of zero.
+__device__ __forceinline__ double fold_fp(const uint32_t *dv, const FpPrime &f) {
+  const uint64_t lo = dv[0] + (static_cast<uint64_t>(dv[1]) << 8) + (static_cast<uint64_t>(dv[2]) << 16);
+  const uint64_t hi = dv[3] + (static_cast<uint64_t>(dv[4]) << 8) + (static_cast<uint64_t>(dv[5]) << 16);
+  return fp_mul(fp_from_word(hi), 16777216.0, 16777216.0 * f.inv_q, f.q) + fp_from_word(lo);
 }
 
 // X = sum_b D_b 2^(8b) of 8 partial sums below 2^24 (byte columns 0-7), as a
