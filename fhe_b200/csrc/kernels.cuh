@@ -57,9 +57,13 @@ unsigned long long kernel_launch_count();
 void unnote_launches(unsigned long long count);
 
 // Launches of one stream follow each other by programmatic dependent launch: the next
-// kernel's CTAs are scheduled as soon as this one's have all started, and wait for its end
-// (and so for every launch before it) in their first instruction, which takes the launch
-// latency between two kernels off the stream: about 2 us each on a chain of small ones.
+// kernel's launch is prepared while this one runs, and its CTAs start as this one's end,
+// waiting for the end of the whole grid (and so for every launch before it) in their first
+// instruction.  That takes the launch latency between two kernels off the stream, about 2 us
+// each on a chain of small ones.  No kernel lets its successor in earlier
+// (griddepcontrol.launch_dependents): waiting CTAs then held places that this kernel's or
+// another stream's could use (a product at N = 2^14 85 us with it, 72 without; a serving
+// batch 10476 and 9954).
 // Every kernel launched this way has to begin with chained_kernel_begin, in every CTA: a
 // grid of which no CTA waits could end before the one before it, and the next one would
 // not wait for that.
@@ -82,7 +86,6 @@ cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, siz
 __device__ __forceinline__ void chained_kernel_begin() {
 #ifdef __CUDA_ARCH__
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #endif
 }
 #endif
