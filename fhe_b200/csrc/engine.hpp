@@ -254,6 +254,8 @@ class Engine {
                                   const Data &to_sparse, const Data &to_dense, int stage_count);
   std::unique_ptr<Data> mod_raise(const Data &ct, const Data &to_sparse, const Data &to_dense);
   std::unique_ptr<Data> multiply_imaginary(const Data &ct, int64_t value);
+  std::unique_ptr<Data> fused_weighted_sum(const std::vector<const Data *> &basis,
+                                           const std::vector<double> &weights);
   std::unique_ptr<Data> weighted_sum(const std::vector<const Data *> &basis,
                                      const std::vector<double> &weights);
   std::vector<std::unique_ptr<Data>> rotate_batch(const Data &ct,

@@ -415,6 +415,19 @@ cudaError_t launch_scalar_rescale(const PrimeTables &t, const KeySwitchTables &k
 cudaError_t launch_to_ntt(const PrimeTables &t, int log_n, int polys, int limbs, int prime_base,
                           const int64_t *x, long long x_stride, int64_t *y, long long y_stride,
                           cudaStream_t s);
+// Terms of a weighted sum of texts of the same limbs: each text's words and the constants of
+// its limbs (as launch_scalar_rescale takes them).
+constexpr int kMaxWeightedTerms = 8;
+struct WeightedTerms {
+  int count = 0;
+  const int64_t *x[kMaxWeightedTerms] = {};
+  LimbScalars c[kMaxWeightedTerms];
+};
+// The sum of the terms' scalar_rescale, added to y where `accumulate` is set.
+cudaError_t launch_weighted_rescale(const PrimeTables &t, const KeySwitchTables &ks, int n, int polys,
+                                    int limbs, int moduli_id, const WeightedTerms &terms, long long x_stride,
+                                    bool accumulate, int64_t *y, long long y_stride, cudaStream_t s);
+
 // to_ntt_ of the rescale of a coefficient-form text in one pass: x is [polys][limbs +
 // 1][N] at src_moduli_id, y is [polys][limbs][N] at src_moduli_id + 1 (NTT form).
 // Limbs outside `exact` are transformed value-only: a word of the same value modulo q, in
