@@ -189,7 +189,7 @@ def kernel_bytes(L: int, E: int, dnum: int, n: int) -> dict:
     return {
         "rescale": (2 * (L + 1) + 2 * L) * limb,          # 2 polys, L+1 -> L limbs
         "to_ntt": 2 * 4 * L * limb,                         # 4 polys in and out
-        "rescale_to_ntt": (2 * (L + 1) + 2 * L) * limb,     # one input: rescaled, NTT
+        "rescale_to_ntt": 2 * (2 * (L + 1) + 2 * L) * limb,  # both inputs: rescaled, NTT
         "tensor_to_intt": (2 * L + L + L) * limb,           # a1, b1 in; d2 out, its own limbs
         "mixed_radix": 2 * L * limb,                        # digits of poly 2
         "mod_up_ntt": (L + up) * limb,                      # digits in, extended out
@@ -911,10 +911,10 @@ def main(argv=None):
         integer, tensor = pipe_figures(prof, args.steps, B, n, L, SPECIAL, clocks.summary()["sm_mhz"],
                                        torch.cuda.get_device_properties(0).multi_processor_count)
         roofline = {"bound": "hbm", "kernel": dominant, "achieved": achieved, "peak": peak,
-                    "limiter": "integer instruction issue: every transform and Montgomery product "
-                               "is 64-bit integer arithmetic on the CUDA cores (integer_pipe); the "
-                               "HBM fraction and the INT8 tensor-pipe fraction (tensor_pipe) are "
-                               "both small",
+                    "limiter": "latency and arithmetic issue: the transforms run on the FP64 pipe "
+                               "(40- and 41-bit primes) and the integer pipes (integer_pipe counts "
+                               "both kinds' butterflies), the base conversions on both and the INT8 "
+                               "tensor pipe (tensor_pipe); the HBM fraction is small",
                     "integer_pipe": integer, "tensor_pipe": tensor,
                     "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                     "peak_source": peak_kind, "avg_launch_ms": avg_ms,
