@@ -91,28 +91,24 @@ __global__ void add_reduce_kernel(PrimeTables t, int n, int limbs, int prime_bas
 
 // -------------------------------------------------------------- rescale --
 
-
-__global__ void rescale_kernel(PrimeTables t, KeySwitchTables ks, int n, int limbs, int moduli_id,
-                               const int64_t *x, long long xs, int64_t *y, long long ys) {
+// grid: (blocks of a limb, output limbs, polynomials), so that a CTA's constants are uniform:
+// 59 rescales at 54-bit primes and N = 2^16 take 1080 us, 1386 to 1464 as a loop over all of
+// a polynomial's words.
+__global__ void __launch_bounds__(kThreads)
+    rescale_kernel(PrimeTables t, KeySwitchTables ks, int n, int moduli_id, const int64_t *x, long long xs,
+                   int64_t *y, long long ys) {
   chained_kernel_begin();
-  const int poly = blockIdx.y;
-  const long long per_poly = static_cast<long long>(limbs - 1) * n;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const int j = blockIdx.y, prime = moduli_id + 1 + j;
+  const int64_t *xp = x + blockIdx.z * xs + c;
+  const int64_t x0 = xp[0], xj = xp[static_cast<long long>(j + 1) * n];
   // get_rounder compares the signed word with the unsigned q/2 (unit.cpp:67-70), so
   // a negative word counts as above it.
-  const uint64_t q_half = t.q[moduli_id] >> 1;
-  const int64_t *xp = x + poly * xs;
-  int64_t *yp = y + poly * ys;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < per_poly;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int j = static_cast<int>(i >> (__ffs(n) - 1));
-    const int c = static_cast<int>(i - static_cast<long long>(j) * n);
-    const int prime = moduli_id + 1 + j;
-    const int64_t x0 = xp[c];
-    const int64_t rounder = static_cast<uint64_t>(x0) > q_half ? 1 : 0;  // get_rounder
-    const long long entry = static_cast<long long>(moduli_id) * ks.prime_count + prime;
-    yp[i] = rescale_word_shoup(xp[static_cast<long long>(j + 1) * n + c], x0, rounder, t.q[prime],
-                               t.k[prime], ks.rescale_scale[entry], ks.rescale_shoup + 2 * entry);
-  }
+  const int64_t rounder = static_cast<uint64_t>(x0) > (t.q[moduli_id] >> 1) ? 1 : 0;
+  const long long entry = static_cast<long long>(moduli_id) * ks.prime_count + prime;
+  y[blockIdx.z * ys + static_cast<long long>(j) * n + c] = rescale_word_shoup(
+      xj, x0, rounder, t.q[prime], t.k[prime], ks.rescale_scale[entry], ks.rescale_shoup + 2 * entry);
 }
 
 // CKKSCore::multiply(ct, double) (core.cpp:196-229) in one pass: every limb entered by
@@ -381,9 +377,10 @@ __global__ void __launch_bounds__(256)
 // term and the bootstrap's NTT-form rotations and diagonal sums end in ModDown), so
 // with every operand in [0, 2^61) the sum is evaluated exactly and reduced to a word
 // in [0, q); otherwise the chain runs term by term.
-__global__ void key_inner_product_kernel(PrimeTables t, DevicePartitions dp, int n, int moduli_id,
-                                         const int64_t *ext, const int64_t *key, int key_primes,
-                                         int view_offset, int64_t *acc) {
+// Five CTAs an SM (48 registers): 13 partitions at N = 2^17 take 708 us, 824 with four.
+__global__ void __launch_bounds__(kThreads, 5)
+    key_inner_product_kernel(PrimeTables t, DevicePartitions dp, int n, int moduli_id, const int64_t *ext,
+                             const int64_t *key, int key_primes, int view_offset, int64_t *acc) {
   chained_kernel_begin();
   const int E = dp.extended;
   const long long total = static_cast<long long>(E) * n;
@@ -447,8 +444,11 @@ __global__ void key_inner_product_kernel(PrimeTables t, DevicePartitions dp, int
 // words are loaded before any is used (the key rows' offsets come with the launch),
 // and one OR of the operands' high words decides between the exact sum and the
 // chain, so the loads of all partitions are in flight together.
+// Four CTAs an SM for one partition (20.7 us a product at N = 2^16 and 6 limbs, 22.9 with
+// three) and for three, the headline's (57.7 us at 27 limbs, for a spill of 28 bytes; without
+// it, at three CTAs, the loads in flight are too few).
 template <int P>
-__global__ void __launch_bounds__(256, P == 3 ? 4 : 0)  // three partitions: 4 CTAs/SM without spills
+__global__ void __launch_bounds__(256, P == 1 || P == 3 ? 4 : 0)
 key_inner_product_fixed_kernel(PrimeTables t, DevicePartitions dp, int log_n, int moduli_id,
                                const int64_t *ext, const int64_t *key, long long poly_row,
                                KeyRowOffsets rows, int64_t *acc, TensorAddend add) {
@@ -632,9 +632,10 @@ cudaError_t launch_add_reduce(const PrimeTables &t, int n, int polys, int limbs,
 cudaError_t launch_rescale(const PrimeTables &t, const KeySwitchTables &ks, int n, int polys,
                            int limbs, int moduli_id, const int64_t *x, long long xs, int64_t *y,
                            long long ys, cudaStream_t s) {
-  const dim3 grid(blocks_for(static_cast<long long>(limbs - 1) * n), polys);
+  if (limbs < 2) return cudaSuccess;  // no limb is left
+  const dim3 grid(blocks_for(n), limbs - 1, polys);
   note_launch();
-  launch_chained(rescale_kernel, grid, kThreads, 0, s, t, ks, n, limbs, moduli_id, x, xs, y, ys);
+  launch_chained(rescale_kernel, grid, kThreads, 0, s, t, ks, n, moduli_id, x, xs, y, ys);
   return cudaGetLastError();
 }
 
