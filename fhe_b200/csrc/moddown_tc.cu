@@ -44,8 +44,8 @@ using namespace umma;
 constexpr int row_bytes(int K) { return (9 * K + 31) / 32 * 32; }  // d_s bytes + sign bytes
 
 // Four CTAs per SM (64 registers) where that costs no spills, fewer otherwise.
-template <int K>
-__global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ? 3 : 1))
+template <int K, bool DOUBLES>
+__global__ void __launch_bounds__(kTcThreads, K <= 10 ? 4 : (K <= 13 ? 3 : 1))
     mod_down_tc_kernel(PrimeTables t, KeySwitchTables ks, ModDownTcTables tc, int n,
                        int moduli_id, int L, const int64_t *acc, EpilogueOps ops, int64_t *out,
                        TcStatus status) {
@@ -84,9 +84,10 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   // 1. Divisor triangle.  From eight special primes on, two adjacent lanes share a
   // coefficient: lane `side` holds the special limbs i = 2 j + side, and each step's divisor
   // comes from its owner by a shuffle; one thread a coefficient left half the warps waiting
-  // at the barrier below and ran a chain twice as long (K = 10: serve_n16 10946 -> 10585 us;
-  // K = 4 with two lanes: eight hoisted rotations 1307 -> 1326 us).  The lanes then write
-  // alternate 16-byte chunks of the A row.
+  // at the barrier below and ran a chain twice as long (K = 10: serving batch 10946 -> 10585
+  // us).  Below, it gains nothing: at K = 6 246.7 us with one lane and 246.2 with two (one
+  // product at N = 2^17), at K = 4 two lanes were slower (eight rotations 1307 -> 1326 us).
+  // The lanes then write alternate 16-byte chunks of the A row.
   constexpr int kLanes = K >= 8 ? 2 : 1;
   if (tid < kTcCoeffs * kLanes) {
     const int c = tid / kLanes, side = tid % kLanes;
@@ -137,7 +138,12 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   const uint32_t tmem = tmem_base;
   const uint32_t bar = smem_addr(&mbar);
 
-  // 2. One MMA round per 16 targets; each thread finishes 8 targets of its coefficient.
+  // 2. One MMA round per 16 targets; each thread finishes 8 targets of its coefficient, two at
+  // a time.  The loop over the pairs is not unrolled and a launch without targets in doubles is
+  // compiled without them: unrolled, the eight copies of both forms' arithmetic and stores
+  // waited on the instruction cache (71 launches of the bootstrap, 54-bit primes: 2282 us
+  // unrolled, 1974 as a loop, 1757 without the doubles; 16 products at N = 2^16: 1008 and
+  // 860 us; eight rotations at K = 4: 309 and 285 us).
   const int lane_base = (warp & 3) * 32;
   const int row = lane_base + lane;
   const int half = warp >> 2;
@@ -150,7 +156,7 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
     const int prime = moduli_id + j;
     const uint64_t q = t.q[prime];
     int64_t v;
-    if (fp_prime(q) && (static_cast<uint64_t>(xj) >> kFpWordBits) == 0) {
+    if (DOUBLES && fp_prime(q) && (static_cast<uint64_t>(xj) >> kFpWordBits) == 0) {
       const FpPrime f{fp_from_word(q), t.inv_q[prime]};
       const double sum = fold_fp(d, f) + fp_mul(fp_from_word(static_cast<uint64_t>(xj)),
                                                 fp_from_word(static_cast<uint64_t>(tc.c_shoup[2 * j])), f);
@@ -160,7 +166,7 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
       fold8(d, lo, hi);
       // REDC(X) < q + 2^19, and x_j prod pinv by Shoup's product is below 2q.  (A plain sum of
       // an fp_prime target whose word is out of range takes one more factor R.)
-      if (fp_prime(q)) {
+      if (DOUBLES && fp_prime(q)) {
         const uint64_t r = static_cast<uint64_t>(redc_wide(lo, hi, q, t.k[prime]));
         lo = static_cast<uint64_t>(mont_mult(static_cast<int64_t>(r), t.r_squared[prime], q, t.k[prime]));
       } else {
@@ -188,10 +194,9 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
     const uint64_t q = t.q[prime];
     const int64_t qs = static_cast<int64_t>(q), q2 = qs << 1;
     if (ops.rescale) {
-      if (j == 0) return;
       const bool up = static_cast<uint64_t>(y0) > q_half;
       const int64_t *shoup = ks.rescale_shoup + 2 * (rescale_row + prime);
-      if (fp_prime(q) && static_cast<uint64_t>(v) < static_cast<uint64_t>(q2) &&
+      if (DOUBLES && fp_prime(q) && static_cast<uint64_t>(v) < static_cast<uint64_t>(q2) &&
           static_cast<uint64_t>(y0) <= static_cast<uint64_t>(q2)) {
         // Both words in the lazy range: the difference's product is canonical.
         const FpPrime f{fp_from_word(q), t.inv_q[prime]};
@@ -228,14 +233,12 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
     }
     // The other buffer's MMAs have completed: every thread passed their wait.
     if (round + 1 < tc.rounds) load_b_round<KB>(sB + ((round + 1) & 1) * kBBytes, tc.b, round + 1);
-    // This thread's words x_j of the round, loaded while the MMAs run.
-    constexpr int kHalfTargets = kTcTargets / 2;
-    int64_t xs[kHalfTargets];
-#pragma unroll
-    for (int u = 0; u < kHalfTargets; u++) {
-      const int j = round * kTcTargets + half * kHalfTargets + u;
-      xs[u] = j < L ? x[static_cast<long long>(j) * n + row] : 0;
-    }
+    // The halves of the CTA take the round's pairs of targets in turn, so that a round of few
+    // targets keeps both busy.  A pair's words x_j are loaded while the MMAs or the pair
+    // before it run.
+    auto target = [&](int pair) { return round * kTcTargets + 4 * pair + 2 * half; };
+    auto word = [&](int j) -> int64_t { return j < L ? x[static_cast<long long>(j) * n + row] : 0; };
+    int64_t xa = word(target(0)), xb = word(target(0) + 1);
     ok = __syncthreads_and(mbar_wait(bar, round & 1, status.wait_limit)) != 0;
     if (!ok) break;
     tc_fence_after();
@@ -243,21 +246,27 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
       if (half == 0) {
         uint32_t d[16];
         tmem_load16(tmem_row, d);
-        first_limb[row] = divided(0, d, xs[0]);
+        first_limb[row] = divided(0, d, xa);
       }
       __syncthreads();
       y0 = first_limb[row];
     }
-#pragma unroll
-    for (int u2 = 0; u2 < kHalfTargets / 2; u2++) {
-      const int jp = half * kHalfTargets + 2 * u2;
-      const int j0 = round * kTcTargets + jp;
-      if (j0 >= L) continue;  // uniform across the warp
+#pragma unroll 1
+    for (int pair = 0; pair < kTcTargets / 4; pair++) {
+      const int j0 = target(pair);
+      if (j0 >= L) break;  // uniform across the warp
       uint32_t d[16];
-      tmem_load16(tmem_row + jp * 8, d);
+      tmem_load16(tmem_row + (j0 - round * kTcTargets) * 8, d);
+      const int64_t xw[2] = {xa, xb};
+      if (pair + 1 < kTcTargets / 4) {
+        xa = word(target(pair + 1));
+        xb = word(target(pair + 1) + 1);
+      }
 #pragma unroll
-      for (int h = 0; h < 2; h++)
-        if (j0 + h < L) put(j0 + h, divided(j0 + h, d + 8 * h, xs[2 * u2 + h]));
+      for (int h = 0; h < 2; h++) {
+        const int j = j0 + h;
+        if (j < L && !(ops.rescale && j == 0)) put(j, divided(j, d + 8 * h, xw[h]));
+      }
     }
     tc_fence_before();
     __syncthreads();
@@ -274,6 +283,28 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 && K != 7 ? 4 : (K <= 13 ?
   __syncthreads();
   tc_fence_after();
   if (warp == 0) tmem_dealloc(tmem);
+}
+
+template <int K, bool DOUBLES>
+cudaError_t launch_tc(dim3 grid, size_t smem, const PrimeTables &t, const KeySwitchTables &ks,
+                      const ModDownTcTables &tc, int n, int moduli_id, int limbs, const int64_t *acc,
+                      const EpilogueOps &ops, int64_t *out, const TcStatus &status, cudaStream_t s) {
+  // The shared-memory limit is raised once per instantiation and device to the most
+  // any supported shape needs, so no attribute call falls inside a graph capture.
+  static int raised = 0;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const int bit = 1 << (device & 31);
+  if (!(raised & bit)) {
+    e = cudaFuncSetAttribute(mod_down_tc_kernel<K, DOUBLES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             200 * 1024);
+    if (e != cudaSuccess) return e;
+    raised |= bit;
+  }
+  note_launch();
+  return launch_chained(mod_down_tc_kernel<K, DOUBLES>, grid, kTcThreads, smem, s, t, ks, tc, n, moduli_id,
+                        limbs, acc, ops, out, status);
 }
 
 size_t tc_smem_bytes(int K) {
@@ -358,33 +389,20 @@ cudaError_t launch_mod_down_epilogue_tc(const PrimeTables &t, const KeySwitchTab
     return cudaErrorInvalidValue;
   const size_t smem = tc_smem_bytes(K);
   const dim3 grid(n / kTcCoeffs, ops.polys);
-  // The shared-memory limit is raised once per instantiation and device to the most
-  // any supported shape needs, so no attribute call falls inside a graph capture.
-  static int raised[17] = {};
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return e;
-  const int bit = 1 << (device & 31);
+  bool doubles = false;
+  for (int j = 0; j < limbs; j++) doubles = doubles || t.fp_primes.has(moduli_id + j);
   switch (K) {
-#define FHE_TC_CASE(KK)                                                                         \
-  case KK:                                                                                      \
-    if (!(raised[KK] & bit)) {                                                                  \
-      e = cudaFuncSetAttribute(mod_down_tc_kernel<KK>,                                          \
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);        \
-      if (e != cudaSuccess) return e;                                                           \
-      raised[KK] |= bit;                                                                        \
-    }                                                                                           \
-    note_launch();                                                                              \
-    launch_chained(mod_down_tc_kernel<KK>, grid, kTcThreads, smem, s, t, ks, tc, n, moduli_id, limbs, acc,  \
-                                                          ops, out, status);                     \
-    break;
+#define FHE_TC_CASE(KK)                                                                                   \
+  case KK:                                                                                                \
+    return doubles                                                                                        \
+               ? launch_tc<KK, true>(grid, smem, t, ks, tc, n, moduli_id, limbs, acc, ops, out, status, s) \
+               : launch_tc<KK, false>(grid, smem, t, ks, tc, n, moduli_id, limbs, acc, ops, out, status, s);
     FHE_TC_CASE(1) FHE_TC_CASE(2) FHE_TC_CASE(3) FHE_TC_CASE(4) FHE_TC_CASE(5) FHE_TC_CASE(6)
     FHE_TC_CASE(7) FHE_TC_CASE(8) FHE_TC_CASE(9) FHE_TC_CASE(10) FHE_TC_CASE(11) FHE_TC_CASE(12)
     FHE_TC_CASE(13) FHE_TC_CASE(14) FHE_TC_CASE(15) FHE_TC_CASE(16)
 #undef FHE_TC_CASE
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 }  // namespace fhe_b200
