@@ -56,6 +56,8 @@ void Engine::check(cudaError_t e, const char *what) {
 }
 
 Engine::Engine(const Config &config) : params(config) {
+  if (params.prime_count > PrimeSet::kPrimes)  // no accepted configuration has as many
+    throw std::invalid_argument("CKKS Parameters: unsupported config.");
   int device = 0;
   check(cudaGetDevice(&device), "cudaGetDevice");
   check(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -105,14 +107,14 @@ Engine::Engine(const Config &config) : params(config) {
       auto plain = [&](int64_t mont) {  // times R^-1
         return static_cast<uint64_t>(guard(mont_exit(mont, qi, ki), static_cast<int64_t>(qi)));
       };
-      if (fp_prime(qi)) tables_.fp_primes.add(i);
+      const bool doubles = fp_prime(qi) && tables_.fp_primes.add(i);
       auto fill = [&](const std::vector<int64_t> &mont, const std::vector<int64_t> &reduced,
                       std::vector<int64_t> &out, int shift) {
         int64_t *o = &out[2 * static_cast<size_t>(i) * p.n];
         const int64_t *in = &reduced[i * per], *word = &mont[i * per];
         for (size_t j = 0; j < per; j++) {
           const uint64_t w = plain(in[j]);
-          if (fp_prime(qi)) {
+          if (doubles) {
             o[j + shift] = static_cast<int64_t>(fp_raw(static_cast<double>(w)));
             o[p.n + j + shift] = static_cast<int64_t>(fp_raw(static_cast<double>(word[j]) * kFpMontScale));
           } else {

@@ -580,10 +580,15 @@ FHE_HD bool redc_operand_ok(int64_t x) {
 }
 
 struct PrimeSet {
-  uint64_t bits[2] = {};  // primes from 128 on are not in it
-  bool has(int prime) const { return prime < 128 && ((bits[prime >> 6] >> (prime & 63)) & 1) != 0; }
-  void add(int prime) {
-    if (prime < 128) bits[prime >> 6] |= uint64_t(1) << (prime & 63);
+  static constexpr int kPrimes = 128;  // what it holds; an engine with more primes is refused
+  uint64_t bits[kPrimes / 64] = {};
+  FHE_HD bool has(int prime) const {
+    return prime < kPrimes && ((bits[prime >> 6] >> (prime & 63)) & 1) != 0;
+  }
+  // Whether the prime is in the set afterwards.
+  bool add(int prime) {
+    if (prime < kPrimes) bits[prime >> 6] |= uint64_t(1) << (prime & 63);
+    return has(prime);
   }
 };
 
@@ -600,7 +605,7 @@ struct PrimeTables {
   const int64_t *root_inverse_reduced;  // root_inverse, each word reduced to [0, q)
   // The same twiddles as (W, W') pairs for shoup_mult: W = root R^-1 mod q, the
   // plain twiddle, and W' = floor(W 2^64 / q); [prime][N][2], entries 0 .. N-2.  A prime
-  // that fp_prime accepts holds two rows of N doubles there instead: W, then the Montgomery
+  // of fp_primes holds two rows of N doubles there instead: W, then the Montgomery
   // word root 2^-62 (fp_mul, fp_mont_mult); twiddle i is entry i + 1 of a forward row and
   // entry i of an inverse one.
   const int64_t *root_shoup;
@@ -611,7 +616,7 @@ struct PrimeTables {
   const int64_t *exit_shoup;
   const double *inv_q;          // 1 / q
   const double *inv_2q;         // 1 / (2q)
-  PrimeSet fp_primes;           // the primes that fp_prime accepts
+  PrimeSet fp_primes;           // the primes that fp_prime accepts: rows of doubles above
   int log_n;
 };
 

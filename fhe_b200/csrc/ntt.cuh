@@ -840,7 +840,8 @@ __device__ __forceinline__ bool ntt_pass_fp(const NttPass &a, const PrimeTables 
 
 // Limbs in the order a pass's CTAs take them: those in integers first, since they take
 // longest and have twice as many CTAs each.
-constexpr int kNttMaxLimbs = 128;  // every preset's chain is shorter
+constexpr int kNttMaxLimbs = PrimeSet::kPrimes;
+static_assert(kNttMaxLimbs <= 256, "limbs are listed as bytes");
 struct NttLimbOrder {
   int integer_limbs = 0;
   uint8_t limb[kNttMaxLimbs] = {};
@@ -904,11 +905,11 @@ __global__ void __launch_bounds__(kNttIntThreads, 4)
       limb < a.skip_start[poly] + a.skip_size[poly])
     return;  // uniform per CTA, before any barrier
   ntt_fold_shape<LOG_N, STRIDED, INVERSE>(a, kNttAllIntTileLog);
-  // A prime that fp_prime accepts has no Shoup pairs: it takes the exact butterflies, whose
+  // A prime with rows of doubles has no Shoup pairs: it takes the exact butterflies, whose
   // words are as good.
   const bool value_limb =
       (VALUE_ONLY == kNttValueOnly || (VALUE_ONLY == kNttMixed && !a.exact.exact(poly, limb))) &&
-      !fp_prime(t.q[a.prime_base + limb]);
+      !t.fp_primes.has(a.prime_base + limb);
   ntt_pass_int<LOG_N, STRIDED, INVERSE, VALUE_ONLY, kNttIntThreads>(a, t, load, store, poly, limb,
                                                                     blockIdx.x, value_limb, tile_smem);
 }
