@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "device_once.hpp"
 #include "modarith.cuh"
 
 namespace fhe_b200 {
@@ -81,6 +82,16 @@ cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, siz
   config.attrs = &attribute;
   config.numAttrs = 1;
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+// Raises a kernel's limit of dynamic shared memory on the current device, the first time.
+template <class Kernel>
+cudaError_t raise_smem_limit(Kernel *kernel, int bytes, DeviceOnce &raised) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess || raised.done(device)) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) raised.set_done(device);
+  return e;
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void chained_kernel_begin() {

@@ -289,19 +289,10 @@ template <int K, bool DOUBLES>
 cudaError_t launch_tc(dim3 grid, size_t smem, const PrimeTables &t, const KeySwitchTables &ks,
                       const ModDownTcTables &tc, int n, int moduli_id, int limbs, const int64_t *acc,
                       const EpilogueOps &ops, int64_t *out, const TcStatus &status, cudaStream_t s) {
-  // The shared-memory limit is raised once per instantiation and device to the most
-  // any supported shape needs, so no attribute call falls inside a graph capture.
-  static int raised = 0;
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
+  // To the most any supported shape needs, so no attribute call falls inside a graph capture.
+  static DeviceOnce raised;
+  const cudaError_t e = raise_smem_limit(mod_down_tc_kernel<K, DOUBLES>, 200 * 1024, raised);
   if (e != cudaSuccess) return e;
-  const int bit = 1 << (device & 31);
-  if (!(raised & bit)) {
-    e = cudaFuncSetAttribute(mod_down_tc_kernel<K, DOUBLES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             200 * 1024);
-    if (e != cudaSuccess) return e;
-    raised |= bit;
-  }
   note_launch();
   return launch_chained(mod_down_tc_kernel<K, DOUBLES>, grid, kTcThreads, smem, s, t, ks, tc, n, moduli_id,
                         limbs, acc, ops, out, status);

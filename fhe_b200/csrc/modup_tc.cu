@@ -214,26 +214,19 @@ cudaError_t launch_mod_up_contract_tc(const PrimeTables &t, const DevicePartitio
   if (!mod_up_tc_supported(dp.max_size, n) || tc.b == nullptr || status.error == nullptr ||
       tc.rounds != (dp.extended + kTcTargets - 1) / kTcTargets)
     return cudaErrorInvalidValue;
-  static int raised[17] = {};
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return e;
-  const int bit = 1 << (device & 31);
+  static DeviceOnce raised[17];
+  cudaError_t e = cudaSuccess;
   const dim3 grid(n / kTcCoeffs, dp.count);
   for (int size = 1; size <= 16; size++) {
     if (!(dp.size_mask & (1u << size))) continue;
     switch (size) {
 #define FHE_UP_CASE(AA)                                                                           \
   case AA:                                                                                        \
-    if (!(raised[AA] & bit)) {                                                                    \
-      e = cudaFuncSetAttribute(mod_up_tc_kernel<AA>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                               static_cast<int>(mod_up_tc_smem(16)));                             \
-      if (e != cudaSuccess) return e;                                                             \
-      raised[AA] |= bit;                                                                          \
-    }                                                                                             \
+    e = raise_smem_limit(mod_up_tc_kernel<AA>, static_cast<int>(mod_up_tc_smem(16)), raised[AA]); \
+    if (e != cudaSuccess) return e;                                                               \
     note_launch();                                                                                \
-    launch_chained(mod_up_tc_kernel<AA>, grid, kTcThreads, mod_up_tc_smem(AA), s, t, dp, tc, n, moduli_id,    \
-                                                                      digits, ext, status, skip_own); \
+    launch_chained(mod_up_tc_kernel<AA>, grid, kTcThreads, mod_up_tc_smem(AA), s, t, dp, tc, n,   \
+                   moduli_id, digits, ext, status, skip_own);                                     \
     break;
       FHE_UP_CASE(1) FHE_UP_CASE(2) FHE_UP_CASE(3) FHE_UP_CASE(4) FHE_UP_CASE(5) FHE_UP_CASE(6)
       FHE_UP_CASE(7) FHE_UP_CASE(8) FHE_UP_CASE(9) FHE_UP_CASE(10) FHE_UP_CASE(11) FHE_UP_CASE(12)

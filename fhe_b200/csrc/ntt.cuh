@@ -944,15 +944,10 @@ cudaError_t launch_ntt_int(const NttPass &a, const PrimeTables &t, const Loader 
   const dim3 grid((1 << a.log_n) >> (a.columns_log + a.stages), a.polys * a.limbs);
   const size_t smem = sizeof(int64_t) << (a.columns_log + a.stages);
   auto kernel = ntt_int_kernel<LOG_N, STRIDED, INVERSE, Loader, Storer, VALUE_ONLY>;
-  // Raised once per instantiation to the most any valid plan uses, so no attribute
-  // call lands inside a graph capture.
-  static bool raised = false;
-  if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kNttMaxSmem);
-    if (e != cudaSuccess) return e;
-    raised = true;
-  }
+  // To the most any valid plan uses, so no attribute call lands inside a graph capture.
+  static DeviceOnce raised;
+  const cudaError_t e = raise_smem_limit(kernel, kNttMaxSmem, raised);
+  if (e != cudaSuccess) return e;
   if (smem > static_cast<size_t>(kNttMaxSmem)) return cudaErrorInvalidValue;
   note_launch(1);
   launch_chained(kernel, grid, kNttIntThreads, smem, stream, a, t, ld, st);

@@ -320,13 +320,12 @@ template <int KIND>
 cudaError_t launch_pass(const TcNttTables &tt, const PrimeTables &t, int polys, int limbs,
                         int prime_base, int64_t *data, long long poly_stride,
                         const TcStatus &status, cudaStream_t s) {
-  static int raised = 0;
-  static int ctas = 0;  // resident CTAs of the whole GPU
+  static DeviceOnce raised;
+  static std::atomic<int> ctas{0};  // resident CTAs of the whole GPU
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return e;
-  const int bit = 1 << (device & 31);
-  if (!(raised & bit)) {
+  if (!raised.done(device)) {
     e = cudaFuncSetAttribute(tc_ntt_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(kSmemBytes));
     // Three CTAs of 66 KB share an SM only with the largest shared-memory carveout.
@@ -338,10 +337,10 @@ cudaError_t launch_pass(const TcNttTables &tt, const PrimeTables &t, int polys, 
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
     ctas = sms * kCtasPerSm;
-    raised |= bit;
+    raised.set_done(device);
   }
   const int total = polys * limbs * (256 / kLines);
-  const int per_cta = (total + ctas - 1) / ctas;
+  const int places = ctas, per_cta = (total + places - 1) / places;
   const int grid = (total + per_cta - 1) / per_cta;
   note_launch();
   tc_ntt_kernel<KIND><<<grid, kTcThreads, kSmemBytes, s>>>(tt, t, data, poly_stride, polys, limbs,
