@@ -99,35 +99,33 @@ Engine::Engine(const Config &config) : params(config) {
     }
     tables_.root_reduced = upload_table(rc);
     tables_.root_inverse_reduced = upload_table(ric);
-    // Plain twiddles with their Shoup quotients (shoup_mult), or as doubles beside the
-    // scaled Montgomery words (fp_prime).
-    std::vector<int64_t> rs(2 * static_cast<size_t>(P) * p.n), ris(rs.size());
-    for (int i = 0; i < P; i++) {
-      const uint64_t qi = p.q[i], ki = p.k[i];
-      auto plain = [&](int64_t mont) {  // times R^-1
-        return static_cast<uint64_t>(guard(mont_exit(mont, qi, ki), static_cast<int64_t>(qi)));
+    for (int i = 0; i < P; i++)
+      if (fp_prime(p.q[i])) tables_.fp_primes.add(i);
+    tables_.root_shoup = upload_table(twiddle_rows(false, tables_.fp_primes));
+    tables_.root_inverse_shoup = upload_table(twiddle_rows(true, tables_.fp_primes));
+    tables_.shoup_tables = &shoup_tables_;
+    shoup_tables_.make = [this] {
+      // (not upload_table: a pending error of the engine is synchronize()'s to report)
+      auto upload = [this](const std::vector<int64_t> &rows) -> const int64_t * {
+        void *d = nullptr;
+        if (cudaMalloc(&d, rows.size() * sizeof(int64_t)) != cudaSuccess) return nullptr;
+        table_buffers_.push_back(static_cast<int64_t *>(d));
+        if (cudaMemcpyAsync(d, rows.data(), rows.size() * sizeof(int64_t), cudaMemcpyHostToDevice, stream_) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(stream_) != cudaSuccess)
+          return nullptr;
+        return static_cast<const int64_t *>(d);
       };
-      const bool doubles = fp_prime(qi) && tables_.fp_primes.add(i);
-      auto fill = [&](const std::vector<int64_t> &mont, const std::vector<int64_t> &reduced,
-                      std::vector<int64_t> &out, int shift) {
-        int64_t *o = &out[2 * static_cast<size_t>(i) * p.n];
-        const int64_t *in = &reduced[i * per], *word = &mont[i * per];
-        for (size_t j = 0; j < per; j++) {
-          const uint64_t w = plain(in[j]);
-          if (doubles) {
-            o[j + shift] = static_cast<int64_t>(fp_raw(static_cast<double>(w)));
-            o[p.n + j + shift] = static_cast<int64_t>(fp_raw(static_cast<double>(word[j]) * kFpMontScale));
-          } else {
-            o[2 * j] = static_cast<int64_t>(w);
-            o[2 * j + 1] = static_cast<int64_t>((static_cast<unsigned __int128>(w) << 64) / qi);
-          }
-        }
-      };
-      fill(p.root, rc, rs, 1);
-      fill(p.root_inverse, ric, ris, 0);
-    }
-    tables_.root_shoup = upload_table(rs);
-    tables_.root_inverse_shoup = upload_table(ris);
+      const int64_t *inverse = upload(twiddle_rows(true, PrimeSet{}));
+      const int64_t *forward = inverse ? upload(twiddle_rows(false, PrimeSet{})) : nullptr;
+      if (forward == nullptr) {
+        cudaGetLastError();  // no memory for them
+        return false;
+      }
+      shoup_tables_.root = forward;
+      shoup_tables_.root_inverse = inverse;
+      return true;
+    };
     // The reduced exit's constant N^-1 R^-1 (n_inverse = N^-1 R) and its Shoup quotient.
     std::vector<int64_t> es(2 * static_cast<size_t>(P));
     for (int i = 0; i < P; i++) {
@@ -226,6 +224,30 @@ Engine::Engine(const Config &config) : params(config) {
   ks_.prime_count = P;
   ks_.special_count = p.special_prime_count;
   seed(nullptr, nullptr);
+}
+
+std::vector<int64_t> Engine::twiddle_rows(bool inverse, const PrimeSet &doubles) const {
+  const size_t n = params.n, per = n - 1;
+  const std::vector<int64_t> &words = inverse ? params.root_inverse : params.root;
+  std::vector<int64_t> rows(2 * n * params.prime_count);
+  for (int i = 0; i < params.prime_count; i++) {
+    const uint64_t q = params.q[i], k = params.k[i];
+    const int64_t *word = &words[i * per];
+    int64_t *row = &rows[2 * n * i];
+    for (size_t j = 0; j < per; j++) {
+      const int64_t reduced = guard(word[j], static_cast<int64_t>(q));
+      const uint64_t w = guard(mont_exit(reduced, q, k), static_cast<int64_t>(q));  // times R^-1
+      if (doubles.has(i)) {
+        const size_t at = inverse ? j : j + 1;
+        row[at] = static_cast<int64_t>(fp_raw(static_cast<double>(w)));
+        row[n + at] = static_cast<int64_t>(fp_raw(static_cast<double>(word[j]) * kFpMontScale));
+      } else {
+        row[2 * j] = static_cast<int64_t>(w);
+        row[2 * j + 1] = static_cast<int64_t>((static_cast<unsigned __int128>(w) << 64) / q);
+      }
+    }
+  }
+  return rows;
 }
 
 Engine::~Engine() {

@@ -368,6 +368,10 @@ class Engine {
   void order_compute_after_upload();    // the compute stream waits for the uploads so far
   std::vector<int64_t *> table_buffers_;
   PrimeTables tables_{};
+  ShoupTables shoup_tables_;
+  // Rows of tables_.root_shoup (or root_inverse_shoup): doubles for the primes in `doubles`,
+  // Shoup pairs for the others.
+  std::vector<int64_t> twiddle_rows(bool inverse, const PrimeSet &doubles) const;
   KeySwitchTables ks_{};
   std::map<std::pair<int, int>, DevicePartitions> partition_cache_;
   int tensor_cores_ = kTensorCoresAuto;

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include "device_once.hpp"
@@ -100,6 +101,21 @@ __device__ __forceinline__ void chained_kernel_begin() {
 #endif
 }
 #endif
+
+// root_shoup and root_inverse_shoup with pairs for every prime, those of fp_primes too: a
+// caller's transform shape runs all limbs in integers.  Made by the first transform that
+// needs them, but not inside a stream capture: the exact butterflies give words as good.
+struct ShoupTables {
+  const int64_t *root = nullptr;
+  const int64_t *root_inverse = nullptr;
+  std::function<bool()> make;  // false: not made
+  bool ready(cudaStream_t stream) {
+    if (root != nullptr) return true;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &capturing) == cudaSuccess &&
+           capturing == cudaStreamCaptureStatusNone && make && make();
+  }
+};
 
 struct KeySwitchTables {
   const int64_t *p_inverse_mult_r;  // [K][P] (entry for prime i at [s*P + i])

@@ -592,6 +592,8 @@ struct PrimeSet {
   }
 };
 
+struct ShoupTables;  // kernels.cuh
+
 // Per-prime constants as the kernels read them.
 struct PrimeTables {
   const uint64_t *q;
@@ -617,6 +619,7 @@ struct PrimeTables {
   const double *inv_q;          // 1 / q
   const double *inv_2q;         // 1 / (2q)
   PrimeSet fp_primes;           // the primes that fp_prime accepts: rows of doubles above
+  ShoupTables *shoup_tables;    // (host) pairs of every prime, for passes in integers
   int log_n;
 };
 

@@ -490,7 +490,10 @@ int fhe_engine_graph_counts(const fhe_engine *engine, int *captured, int *failed
  * contiguous pass covers s_second stages, the strided pass log_n - s_second;
  * 2^first_columns_log sub-transforms share a CTA in the strided pass and
  * 2^second_tile_log words make a CTA tile in the contiguous one.  Every shape gives
- * the same words; fhe_b200/autotune.py measures them on the device and writes the
+ * the same words, but only the default shapes compute the limbs of 40- and 41-bit primes in
+ * doubles; any other runs all limbs in integers, which takes 1.5 to 2 times as long, and
+ * an engine's first product or key switch under it makes tables for that (32 N bytes a
+ * prime).  fhe_b200/autotune.py measures the shapes on the device and writes the
  * fastest to fhe_b200/ntt_tuning.json, which the Python package installs on load.
  * set returns FHE_ERR_INVALID_ARGUMENT for a shape the kernels cannot run. */
 int fhe_ntt_tuning_set(int log_n, int s_second, int first_columns_log, int second_tile_log);
