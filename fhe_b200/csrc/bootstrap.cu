@@ -206,12 +206,13 @@ std::unique_ptr<Data> Engine::multiply_imaginary(const Data &ct, int64_t value) 
 std::unique_ptr<Data> Engine::fused_weighted_sum(const std::vector<const Data *> &basis,
                                                  const std::vector<double> &weights) {
   // The products by scalars and their sums (multiply_scalar, add) where they are limb by
-  // limb: coefficient-form, unrescaled texts of one level whose products' scales match.
-  // Otherwise null, and the caller takes them one at a time.
+  // limb: coefficient-form, unrescaled texts of one level whose products' scales match, as
+  // many as a launch takes (the sine's series has at most seven).  Otherwise null, and the
+  // caller takes them one at a time.
   std::vector<int> used;  // in the reference's order
   for (int i = static_cast<int>(weights.size()) - 1; i > 0; i--)
     if (weights[i] != 0) used.push_back(i);
-  if (used.size() < 2) return nullptr;
+  if (used.size() < 2 || used.size() > static_cast<size_t>(kMaxWeightedTerms)) return nullptr;
   const Data &first = *basis[used[0] - 1];
   const int level = first.level(), mid = first.moduli_id, L = first.chains;
   if ((first.polys != 2 && first.polys != 3) || level <= 0 || L < 2 || L > kMaxScalarLimbs) return nullptr;
@@ -227,21 +228,18 @@ std::unique_ptr<Data> Engine::fused_weighted_sum(const std::vector<const Data *>
     flag |= x.flag;
   }
   auto out = make_data(kUnitCiphertext, flag, params.moduli_id(level - 1), first.polys, scale);
-  for (size_t at = 0; at < used.size(); at += kMaxWeightedTerms) {
-    WeightedTerms terms;
-    for (size_t i = at; i < used.size() && terms.count < kMaxWeightedTerms; i++) {
-      const auto mult = mult_multiplier(weights[used[i]], level);
-      terms.x[terms.count] = basis[used[i] - 1]->d;
-      LimbScalars &c = terms.c[terms.count++];
-      c = LimbScalars{};
-      for (int j = 0; j < L; j++) c.v[j] = mult[j];
-    }
-    check(timed("scalar_rescale", [&] {
-            return launch_weighted_rescale(tables_, ks_, params.n, first.polys, L, mid, terms, first.poly_stride(),
-                                           at > 0, out->d, out->poly_stride(), stream_);
-          }),
-          "weighted sum");
+  WeightedTerms terms;
+  for (int i : used) {
+    const auto mult = mult_multiplier(weights[i], level);
+    terms.x[terms.count] = basis[i - 1]->d;
+    LimbScalars &c = terms.c[terms.count++];
+    for (int j = 0; j < L; j++) c.v[j] = mult[j];
   }
+  check(timed("scalar_rescale", [&] {
+          return launch_weighted_rescale(tables_, ks_, params.n, first.polys, L, mid, terms, first.poly_stride(),
+                                         out->d, out->poly_stride(), stream_);
+        }),
+        "weighted sum");
   return out;
 }
 

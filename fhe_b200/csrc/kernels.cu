@@ -148,12 +148,12 @@ __global__ void scalar_rescale_kernel(PrimeTables t, KeySwitchTables ks, int log
 
 // y = sum over the terms of scalar_rescale_kernel's words (each term's text entered by its
 // constants and rescaled), added as mont_add_reduce_2q_to_q adds canonical words, whose order
-// does not matter; `accumulate` starts from y.  One launch in place of a product and a sum a
-// term: the products are not written and read again.
+// does not matter.  One launch in place of a product and a sum a term: the products are not
+// written and read again.
 __global__ void __launch_bounds__(kThreads)
     weighted_rescale_kernel(PrimeTables t, KeySwitchTables ks, int log_n, int limbs, int moduli_id,
-                            const __grid_constant__ WeightedTerms terms, long long xs, bool accumulate,
-                            int64_t *y, long long ys) {
+                            const __grid_constant__ WeightedTerms terms, long long xs, int64_t *y,
+                            long long ys) {
   chained_kernel_begin();
   const int poly = blockIdx.z;
   const long long cidx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -161,10 +161,7 @@ __global__ void __launch_bounds__(kThreads)
   const uint64_t q0 = t.q[moduli_id], k0 = t.k[moduli_id];
   int64_t *yp = y + poly * ys + cidx;
   const int j0 = blockIdx.y * kScalarLimbsPerThread;
-  int64_t sum[kScalarLimbsPerThread];
-#pragma unroll
-  for (int u = 0; u < kScalarLimbsPerThread; u++)
-    sum[u] = accumulate && j0 + u < limbs - 1 ? yp[static_cast<long long>(j0 + u) << log_n] : 0;
+  int64_t sum[kScalarLimbsPerThread] = {};
   for (int m = 0; m < terms.count; m++) {
     const int64_t *xp = terms.x[m] + poly * xs + cidx;
     int64_t x[kScalarLimbsPerThread];
@@ -185,7 +182,7 @@ __global__ void __launch_bounds__(kThreads)
       const long long entry = static_cast<long long>(moduli_id) * ks.prime_count + prime;
       const int64_t v = rescale_word_shoup(ej, e0, rounder, q, k, ks.rescale_scale[entry],
                                            ks.rescale_shoup + 2 * entry);
-      sum[u] = !accumulate && m == 0 ? v : guard(guard(sum[u] + v, qs << 1), qs);
+      sum[u] = m == 0 ? v : guard(guard(sum[u] + v, qs << 1), qs);
     }
   }
 #pragma unroll
@@ -655,14 +652,14 @@ cudaError_t launch_scalar_rescale(const PrimeTables &t, const KeySwitchTables &k
 
 cudaError_t launch_weighted_rescale(const PrimeTables &t, const KeySwitchTables &ks, int n, int polys,
                                     int limbs, int moduli_id, const WeightedTerms &terms, long long x_stride,
-                                    bool accumulate, int64_t *y, long long y_stride, cudaStream_t s) {
+                                    int64_t *y, long long y_stride, cudaStream_t s) {
   if (limbs < 2 || limbs > kMaxScalarLimbs || terms.count < 1 || terms.count > kMaxWeightedTerms)
     return cudaErrorInvalidValue;
   const int log_n = __builtin_ctz(static_cast<unsigned>(n));
   const dim3 grid(blocks_for(n), (limbs - 1 + kScalarLimbsPerThread - 1) / kScalarLimbsPerThread, polys);
   note_launch();
   return launch_chained(weighted_rescale_kernel, grid, kThreads, 0, s, t, ks, log_n, limbs, moduli_id, terms,
-                        x_stride, accumulate, y, y_stride);
+                        x_stride, y, y_stride);
 }
 
 cudaError_t launch_mixed_radix(const PrimeTables &t, const DevicePartitions &dp, int n,

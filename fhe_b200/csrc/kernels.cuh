@@ -450,10 +450,10 @@ struct WeightedTerms {
   const int64_t *x[kMaxWeightedTerms] = {};
   LimbScalars c[kMaxWeightedTerms];
 };
-// The sum of the terms' scalar_rescale, added to y where `accumulate` is set.
+// The sum of the terms' scalar_rescale.
 cudaError_t launch_weighted_rescale(const PrimeTables &t, const KeySwitchTables &ks, int n, int polys,
                                     int limbs, int moduli_id, const WeightedTerms &terms, long long x_stride,
-                                    bool accumulate, int64_t *y, long long y_stride, cudaStream_t s);
+                                    int64_t *y, long long y_stride, cudaStream_t s);
 
 // to_ntt_ of the rescale of a coefficient-form text in one pass: x is [polys][limbs +
 // 1][N] at src_moduli_id, y is [polys][limbs][N] at src_moduli_id + 1 (NTT form).
