@@ -196,10 +196,11 @@ __global__ void __launch_bounds__(kThreads)
 // perhaps the last: the digits after the first are canonical residues (each is reduced to
 // [0, q) from a value in the lazy range), so any exact evaluation gives them.  Here a digit
 // is (x_j - Y_j) inverse_j in doubles (modarith.cuh), Y_j = x_0 + sum_i y_i product_ij kept
-// unreduced: a term is within 3/4 q of zero, so |Y_j| stays below 9 q and x_j - Y_j below
-// 2^45.  A last limb of another prime takes its Y as integers.  False where a word is
-// outside [0, 2q_j) or the first one outside [0, 2 q_j] for some j: the reference's steps are
-// then not canonical, and the caller takes them as written.
+// unreduced: x_0 is at most 2 q_j and each of up to A - 2 terms within 3/4 q_j of zero, so
+// |Y_j| is at most (2 + 3/4 (A - 2)) q_j <= 12.5 q_j for A <= 16 and x_j - Y_j, below 14.5 q_j
+// with q_j < 2^41, below 2^45.  A last limb of another prime takes its Y as integers.  False
+// where a word is outside [0, 2q_j) or the first one outside [0, 2 q_j] for some j: the
+// reference's steps are then not canonical, and the caller takes them as written.
 template <int A>
 __device__ __forceinline__ bool garner_fp(const PrimeTables &t, const DevicePartitions &dp, int p, int prime0,
                                           const int64_t (&xw)[A], int64_t (&y)[A]) {
@@ -249,10 +250,13 @@ __device__ __forceinline__ bool garner_fp(const PrimeTables &t, const DevicePart
 
 // One partition of alpha = A limbs per thread-coefficient (rns_to_mrs,
 // core_key_switch.cpp:21-56, Garner's algorithm with the reference's lazy ranges).
-// Six CTAs per SM where the digits fit the registers that leaves (A <= 10).
+// Six CTAs an SM where the digits fit the 80 registers that leaves (A <= 7), five up to ten
+// limbs: at six those spilled 12 to 60 bytes (16 products at N = 2^16, partitions of 7 and 10
+// limbs: 395 us, 380 with five).  At four the largest (13 to 16) spill up to 128 bytes, but
+// were slower at three without (16 limbs: 27.0 us a product, 31.1).
 constexpr int kMixedRadixThreads = 128;
 template <int A>
-__global__ void __launch_bounds__(kMixedRadixThreads, A <= 10 ? 6 : 4)
+__global__ void __launch_bounds__(kMixedRadixThreads, A <= 7 ? 6 : (A <= 10 ? 5 : 4))
     mixed_radix_kernel(PrimeTables t, DevicePartitions dp, int n, int moduli_id,
                                    const int64_t *x, int64_t *digits) {
   chained_kernel_begin();
