@@ -244,12 +244,16 @@ int fhe_conjugate_plaintext(fhe_engine *engine, const fhe_data *pt, fhe_data **o
  * core_encode.cpp:33-150): `count` slot values (im NULL: real input; fewer than the
  * slot count are zero-padded, more are ignored) encoded at `level` into a plaintext
  * in coefficient form.  The FFT, twist and rounding run on the device in IEEE
- * double with the reference's operation order, so the limbs are bit-identical. */
+ * double with the reference's operation order, so the limbs are bit-identical.  The
+ * values are copied to pinned memory of the engine, so the caller's arrays are free when
+ * the call returns; inside a stream capture, whose replay would read that memory later,
+ * the call is refused (FHE_ERR_CUDA) and the capture stays valid. */
 int fhe_encode(fhe_engine *engine, const double *re, const double *im, int count, int level,
                int include_special, fhe_data **out);
 /* CKKSEngine::decode_unit / decode_complex_unit_plaintext (engine.h:75-77,
  * engine_decode.cpp:6-19; core_decode.cpp:11-124): slot_count values into re (and
- * im unless NULL).  CRT reconstruction, skew, FFT and permutation run on the device. */
+ * im unless NULL).  CRT reconstruction, skew, FFT and permutation run on the device.
+ * The call waits for the engine's work, so it cannot run inside a stream capture. */
 int fhe_decode(fhe_engine *engine, const fhe_data *pt, double *re, double *im);
 
 /* ---- arithmetic (engine_add.cpp, engine_subtract.cpp, engine_multiply.cpp,

@@ -46,3 +46,30 @@ def test_encode_pads_short_inputs_with_zeros(engines):
     a = e.encode(short, 3).download()
     b = e.encode(padded, 3).download()
     assert np.array_equal(a, b)
+
+
+def test_encode_is_refused_inside_a_capture(engines):
+    import torch
+
+    from fhe_b200 import FheError
+
+    e = engines(14, 1, 1)
+    values = np.linspace(-1, 1, 300)
+    want = e.encode(values, 3).download()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    total = torch.zeros(1, device="cuda")
+    torch.cuda.synchronize()
+    e.set_stream(stream.cuda_stream)
+    try:
+        with torch.cuda.graph(graph, stream=stream):
+            total += 1
+            with pytest.raises(FheError, match="stream capture"):
+                e.encode(values, 3)
+            total += 1
+        graph.replay()  # the capture stayed valid
+        torch.cuda.synchronize()
+        assert total.item() == 2
+        assert np.array_equal(e.encode(values, 3).download(), want)
+    finally:
+        torch.cuda.synchronize()
+        e.set_stream(None)
