@@ -14,7 +14,7 @@ def residues(values, moduli):
 
 @pytest.mark.parametrize("log_n,special,limb_counts", [
     (13, 1, (2, 3, 4)), (16, 10, (2, 5, 11, 29)),
-    (17, 6, (2, 3, 4, 5, 6, 8, 11, 13, 15, 20, 25, 31, 40, 47)),
+    (17, 6, (2, 3, 4, 5, 6, 7, 8, 11, 13, 15, 16, 19, 20, 25, 31, 40, 47)),
 ])
 def test_the_limb_count_does_not_change_the_slots(engines, log_n, special, limb_counts):
     e = engines(log_n, special, 1)
@@ -32,15 +32,17 @@ def test_the_limb_count_does_not_change_the_slots(engines, log_n, special, limb_
     for s in slots[1:]:
         assert np.array_equal(s, slots[0])
     # Integers near Q / 2 and Q / 3 as constant polynomials: every slot has their value, the
-    # sign past Q / 2 negative.  The words are summed in doubles: one rounding a word.
+    # sign past Q / 2 negative.  The words are summed in doubles: one rounding a word.  Where
+    # those exceed a double's range (more than 25 limbs), powers of two within it.
     for limbs in limb_counts:
         q = [int(v) for v in e.moduli[e.chain_count - limbs:e.chain_count]]
-        if limbs > 16:
-            continue  # 2^(64 w) overflows past w = 15, as in the reference
         big = 1
         for v in q:
             big *= v
-        for m in (big // 2 - 1, big // 2 + 1, big // 3, big - big // 3):
+        values = (big // 2 - 1, big // 2 + 1, big // 3, big - big // 3)
+        if big.bit_length() > 1023:  # 2^(64 w) overflows past w = 15, as in the reference
+            values = (1, big - 1, 2 ** 1000, big - 2 ** 1000)
+        for m in values:
             x = np.zeros((1, limbs, e.coeff_count), dtype=np.int64)
             x[:, :, :1] = residues([m], q)
             got = e.decode(e.upload(x, e.chain_count - limbs, kind=PLAINTEXT))

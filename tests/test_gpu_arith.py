@@ -1,10 +1,11 @@
 """GPU parity of ciphertext arithmetic: additions, subtractions, plaintext and
 scalar products, negation and squaring through the C ABI, against the reference's
 engine on the same operands (level matching, rescale state and NTT form included)."""
+import numpy as np
 import pytest
 
 from conftest import load_golden
-from inputs import arith_inputs, digest
+from inputs import arith_inputs, digest, uniform_limbs
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +58,25 @@ def test_arithmetic_matches_recorded_reference(engines, case):
         if digest(out.download()) != want:
             failures.append(key)
     assert not failures, failures
+
+
+@pytest.mark.parametrize("log_n,special,preset,limbs", [(13, 1, 1, 3), (14, 1, 1, 6), (15, 2, 1, 17), (16, 4, 2, 9)])
+def test_a_plaintext_times_three_polynomials(engines, log_n, special, preset, limbs):
+    """Text and plaintext of one level are rescaled and transformed in one launch, whatever
+    the text's number of polynomials: each polynomial's product is that of a two-polynomial
+    text (recorded from the reference above) with it in either place."""
+    from fhe_b200 import UNIT_PLAINTEXT
+
+    e = engines(log_n, special, preset)
+    mid = e.chain_count - limbs
+    rng = np.random.default_rng(31 * log_n + limbs)
+    q = e.moduli[mid:e.chain_count]
+    x, plain = uniform_limbs(rng, q, 3, e.coeff_count), uniform_limbs(rng, q, 1, e.coeff_count)
+    pt = e.upload(plain, mid, kind=UNIT_PLAINTEXT)
+    three = e.multiply_plaintext(e.upload(x, mid), pt).download()
+    assert three.shape[0] == 3
+    assert np.array_equal(three[:2], e.multiply_plaintext(e.upload(x[:2], mid), pt).download())
+    assert np.array_equal(three[[2, 1]], e.multiply_plaintext(e.upload(x[[2, 1]], mid), pt).download())
+    product = e.multiply_plaintext(e.ntt(e.upload(x, mid)), e.ntt(pt)).download()  # one text at a time
+    low = np.asarray(q[1:], dtype=np.int64)[None, :, None]
+    assert np.array_equal(product % low, three % low)
