@@ -66,20 +66,25 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 ? 4 : (K <= 13 ? 3 : 1))
   const int64_t *x = acc + static_cast<long long>(poly) * (L + K) * n + coeff0;
 
   load_b_round<KB>(sB, tc.b, 0);
-  // The triangle's constants, read at fixed offsets (entries past a step's limbs are zero);
-  // from the tables each product took three loads and their addresses (16 products at
-  // N = 2^16: 5730 us, 5441 with the copy).
-  __shared__ uint64_t special_q[K], special_k[K];
-  __shared__ int64_t special_inverse[K * K];
-  for (int i = tid; i < K * K; i += kTcThreads) {
-    const int s = i / K, limb = i % K;
-    special_inverse[i] = limb < K - 1 - s ? ks.p_inverse_mult_r[s * P + moduli_id + L + limb] : 0;
-    if (i < K) {
-      special_q[i] = t.q[moduli_id + L + i];
-      special_k[i] = t.k[moduli_id + L + i];
+  // The triangle's constants in shared memory from eight special primes on, read at fixed
+  // offsets (entries past a step's limbs are zero): from the tables each product takes three
+  // loads and their addresses (K = 10: 16 products at N = 2^16 893 us, 864 with the copy).
+  // Below, the copy and its barrier cost more than they give (K = 4: eight rotations 277 us,
+  // 286 with it).
+  constexpr bool kCopy = K >= 8;
+  __shared__ uint64_t special_q[kCopy ? K : 1], special_k[kCopy ? K : 1];
+  __shared__ int64_t special_inverse[kCopy ? K * K : 1];
+  if (kCopy) {
+    for (int i = tid; i < K * K; i += kTcThreads) {
+      const int s = i / K, limb = i % K;
+      special_inverse[i] = limb < K - 1 - s ? ks.p_inverse_mult_r[s * P + moduli_id + L + limb] : 0;
+      if (i < K) {
+        special_q[i] = t.q[moduli_id + L + i];
+        special_k[i] = t.k[moduli_id + L + i];
+      }
     }
+    __syncthreads();
   }
-  __syncthreads();
 
   // 1. Divisor triangle.  From eight special primes on, two adjacent lanes share a
   // coefficient: lane `side` holds the special limbs i = 2 j + side, and each step's divisor
@@ -112,10 +117,11 @@ __global__ void __launch_bounds__(kTcThreads, K <= 10 ? 4 : (K <= 13 ? 3 : 1))
       for (int j = 0; j < kOwn; j++) {
         if (kLanes * j >= K - 1 - s) continue;
         const int i = kLanes * j + side;  // the odd lane may have none left: its product is dropped
-        const uint64_t q = special_q[i < K ? i : K - 1];
+        const int limb = i < K ? i : K - 1, prime = moduli_id + L + limb;
+        const uint64_t q = kCopy ? special_q[limb] : t.q[prime];
         const int64_t q2 = static_cast<int64_t>(q << 1);
-        const int64_t v = mont_mult_const(special_inverse[s * K + i], guard(sp[j] + q2 - d, q2), q,
-                                          special_k[i < K ? i : K - 1]);
+        const int64_t v = mont_mult_const(kCopy ? special_inverse[s * K + limb] : ks.p_inverse_mult_r[s * P + prime],
+                                          guard(sp[j] + q2 - d, q2), q, kCopy ? special_k[limb] : t.k[prime]);
         sp[j] = i < K - 1 - s ? v : sp[j];
       }
     }
