@@ -674,7 +674,10 @@ cudaError_t launch_mixed_radix(const PrimeTables &t, const DevicePartitions &dp,
     if (!(dp.size_mask & (1u << size))) continue;
     switch (size) {
 #define FHE_MRS_CASE(A) \
-  case A: note_launch(); launch_chained(mixed_radix_kernel<A>, grid, kMixedRadixThreads, 0, s, t, dp, n, moduli_id, x, digits); break;
+  case A:                                                                                              \
+    note_launch();                                                                                     \
+    launch_chained(mixed_radix_kernel<A>, grid, kMixedRadixThreads, 0, s, t, dp, n, moduli_id, x, digits); \
+    break;
       FHE_MRS_CASE(1) FHE_MRS_CASE(2) FHE_MRS_CASE(3) FHE_MRS_CASE(4) FHE_MRS_CASE(5)
       FHE_MRS_CASE(6) FHE_MRS_CASE(7) FHE_MRS_CASE(8) FHE_MRS_CASE(9) FHE_MRS_CASE(10)
       FHE_MRS_CASE(11) FHE_MRS_CASE(12) FHE_MRS_CASE(13) FHE_MRS_CASE(14) FHE_MRS_CASE(15)
@@ -741,7 +744,7 @@ cudaError_t launch_key_inner_product(const PrimeTables &t, const DevicePartition
     return cudaGetLastError();
   }
   note_launch();
-  launch_chained(key_inner_product_kernel, blocks_for(static_cast<long long>(dp.extended) * n), kThreads, 0, s, 
+  launch_chained(key_inner_product_kernel, blocks_for(static_cast<long long>(dp.extended) * n), kThreads, 0, s,
       t, dp, n, moduli_id, ext, key, key_primes, view_offset, acc);
   return cudaGetLastError();
 }

@@ -339,7 +339,7 @@ void Engine::draw_uniform(int64_t *out, long long row_stride, int rows, int prim
                           uint64_t fixed_max, int64_t shift) {
   const long long blocks = (static_cast<long long>(params.n) >> 2) * rows;
   note_launch();
-  launch_chained(rng_uniform_kernel, grid_for(blocks), kThreads, 0, stream_, 
+  launch_chained(rng_uniform_kernel, grid_for(blocks), kThreads, 0, stream_,
       rng_, rng_counter_, params.log_n, rows, tables_.q, prime_base, fixed_max, shift, out,
       row_stride);
   rng_counter_ += static_cast<unsigned long long>(blocks);
@@ -386,7 +386,7 @@ void Engine::encrypt_finish(int polys, int limbs, int prime_base, bool subtract,
 
 void Engine::tile(const int64_t *chain, int limbs, int prime_base, int64_t *y, long long y_stride) {
   note_launch();
-  launch_chained(tile_kernel, grid_for(static_cast<long long>(limbs) << params.log_n), kThreads, 0, stream_, 
+  launch_chained(tile_kernel, grid_for(static_cast<long long>(limbs) << params.log_n), kThreads, 0, stream_,
       tables_, params.log_n, limbs, prime_base, chain, y, y_stride);
   check(cudaGetLastError(), "tile");
 }
@@ -394,8 +394,8 @@ void Engine::tile(const int64_t *chain, int limbs, int prime_base, int64_t *y, l
 void Engine::signed_tile(const int64_t *chain, int64_t q_src, int limbs, int prime_base,
                          int64_t *y, long long y_stride) {
   note_launch();
-  launch_chained(signed_tile_kernel, grid_for(static_cast<long long>(limbs) << params.log_n), kThreads, 0, stream_, tables_, params.log_n, limbs, prime_base, chain, q_src, y,
-                                  y_stride);
+  launch_chained(signed_tile_kernel, grid_for(static_cast<long long>(limbs) << params.log_n), kThreads, 0,
+                 stream_, tables_, params.log_n, limbs, prime_base, chain, q_src, y, y_stride);
   check(cudaGetLastError(), "signed tile");
 }
 
@@ -415,10 +415,10 @@ void Engine::pointwise(int op, int limbs, int prime_base, const int64_t *a, cons
   check(timed("pointwise", [&] {
           note_launch();
           if (aligned && params.n >= 4)
-            launch_chained(pointwise_kernel<4>, grid_for(words / 4), kThreads, 0, stream_, 
+            launch_chained(pointwise_kernel<4>, grid_for(words / 4), kThreads, 0, stream_,
                 tables_, op, params.log_n, limbs, period, prime_base, a, b, c, y);
           else
-            launch_chained(pointwise_kernel<1>, grid_for(words), kThreads, 0, stream_, 
+            launch_chained(pointwise_kernel<1>, grid_for(words), kThreads, 0, stream_,
                 tables_, op, params.log_n, limbs, period, prime_base, a, b, c, y);
           return cudaGetLastError();
         }),

@@ -980,7 +980,8 @@ cudaError_t launch_ntt_pass(const NttPass &a, bool standard, bool integer, const
   switch (a.log_n) {
 #define FHE_NTT_CASE(L)                                                               \
   case L:                                                                             \
-    launch_chained(ntt_pass_kernel<L, STRIDED, INVERSE, Loader, Storer, VALUE_ONLY>, blocks, kNttThreads, 0, stream, a, order, t, ld, st);                    \
+    launch_chained(ntt_pass_kernel<L, STRIDED, INVERSE, Loader, Storer, VALUE_ONLY>,  \
+                   blocks, kNttThreads, 0, stream, a, order, t, ld, st);              \
     break;
     FHE_NTT_CASE(13) FHE_NTT_CASE(14) FHE_NTT_CASE(15) FHE_NTT_CASE(16) FHE_NTT_CASE(17)
 #undef FHE_NTT_CASE

@@ -14,14 +14,16 @@ cudaError_t launch_rescale_to_ntt(const PrimeTables &t, const KeySwitchTables &k
   const long long row = static_cast<long long>(src_moduli_id) * ks.prime_count;
   PlainStore st{y, y_stride};
   if (exact.poly == ExactLimbs::kAllExact) {
-    RescaleEnterLoad<false> ld{x, x_stride, first_polys, second, src_moduli_id, ks.rescale_scale + row, ks.rescale_shoup + 2 * row,
-                               t.r_squared, t.q, t.k, t.r_mod, ks.rescale_enter_shoup + 2 * row, exact};
+    RescaleEnterLoad<false> ld{x, x_stride, first_polys, second, src_moduli_id, ks.rescale_scale + row,
+                               ks.rescale_shoup + 2 * row, t.r_squared, t.q, t.k, t.r_mod,
+                               ks.rescale_enter_shoup + 2 * row, exact};
     // A 60-bit dropped prime's words are too wide for the exact form in doubles.
     return forward_ntt(log_n, polys, limbs, src_moduli_id + 1, t, ld, st, y, y_stride, s, nullptr, nullptr,
                        ExactLimbs{}, !t.fp_primes.has(src_moduli_id));
   }
-  RescaleEnterLoad<true> ld{x, x_stride, first_polys, second, src_moduli_id, ks.rescale_scale + row, ks.rescale_shoup + 2 * row,
-                            t.r_squared, t.q, t.k, t.r_mod, ks.rescale_enter_shoup + 2 * row, exact};
+  RescaleEnterLoad<true> ld{x, x_stride, first_polys, second, src_moduli_id, ks.rescale_scale + row,
+                            ks.rescale_shoup + 2 * row, t.r_squared, t.q, t.k, t.r_mod,
+                            ks.rescale_enter_shoup + 2 * row, exact};
   return forward_ntt<RescaleEnterLoad<true>, PlainStore, kNttMixed>(
       log_n, polys, limbs, src_moduli_id + 1, t, ld, st, y, y_stride, s, nullptr, nullptr, exact);
 }

@@ -119,7 +119,7 @@ cudaError_t launch_tensor_to_intt(const PrimeTables &t, int log_n, int limbs, in
   if (third_only && log_n >= 9 && aligned) {
     // d2 first, then a plain mixed inverse transform in place.
     note_launch();
-    launch_chained(tensor_third_kernel, blocks_for(static_cast<long long>(limbs) << (log_n - 1)), kThreads, 0, s, 
+    launch_chained(tensor_third_kernel, blocks_for(static_cast<long long>(limbs) << (log_n - 1)), kThreads, 0, s,
         t, ld, log_n, limbs, prime_base, y);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

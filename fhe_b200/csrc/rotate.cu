@@ -228,7 +228,7 @@ cudaError_t launch_permute_signed(const PrimeTables &t, int n, int polys, int li
   if (x == y) return cudaErrorInvalidValue;  // a scatter cannot run in place
   const int log_n = __builtin_ctz(static_cast<unsigned>(n));
   note_launch();
-  launch_chained(permute_signed_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, s, 
+  launch_chained(permute_signed_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, s,
       t, log_n, polys, limbs, prime_base, x, x_stride, signed_perm, y, y_stride);
   return cudaGetLastError();
 }
@@ -239,7 +239,7 @@ cudaError_t launch_permute_gather(int n, int polys, int limbs, const int64_t *x,
   if (x == y) return cudaErrorInvalidValue;
   const int log_n = __builtin_ctz(static_cast<unsigned>(n));
   note_launch();
-  launch_chained(permute_gather_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, s, 
+  launch_chained(permute_gather_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, s,
       log_n, polys, limbs, x, x_stride, perm, y, y_stride);
   return cudaGetLastError();
 }
@@ -251,7 +251,7 @@ cudaError_t launch_scalar_enter(const PrimeTables &t, int n, int polys, int limb
   if (limbs > kMaxScalarLimbs) return cudaErrorInvalidValue;
   const int log_n = __builtin_ctz(static_cast<unsigned>(n));
   note_launch();
-  launch_chained(scalar_enter_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, st, 
+  launch_chained(scalar_enter_kernel, grid_for(static_cast<long long>(polys) * limbs * n), kThreads, 0, st,
       t, log_n, polys, limbs, prime_base, x, x_stride, x_limb_offset, s, y, y_stride);
   return cudaGetLastError();
 }
@@ -260,7 +260,7 @@ cudaError_t launch_ntt_rotate_finish(const PrimeTables &t, int log_n, int limbs,
                                      const int64_t *x0, const int64_t *acc, const int32_t *perm,
                                      int64_t *y, cudaStream_t s) {
   note_launch();
-  launch_chained(ntt_rotate_finish_kernel, grid_for((2LL * limbs) << log_n), kThreads, 0, s, 
+  launch_chained(ntt_rotate_finish_kernel, grid_for((2LL * limbs) << log_n), kThreads, 0, s,
       t, log_n, limbs, prime_base, x0, acc, perm, y);
   return cudaGetLastError();
 }
@@ -275,10 +275,10 @@ cudaError_t launch_diagonal_mac(const PrimeTables &t, int log_n, int limbs, int 
     bits |= reinterpret_cast<uintptr_t>(terms.x[m]) | reinterpret_cast<uintptr_t>(terms.d[m]);
   note_launch();
   if ((bits & 15) == 0 && log_n >= 1)
-    launch_chained(diagonal_mac_kernel<2>, grid_for(((2LL * limbs) << log_n) / 2), kThreads, 0, s, 
+    launch_chained(diagonal_mac_kernel<2>, grid_for(((2LL * limbs) << log_n) / 2), kThreads, 0, s,
         t, log_n, limbs, prime_base, terms, x_stride, accumulate, y, y_stride);
   else
-    launch_chained(diagonal_mac_kernel<1>, grid_for((2LL * limbs) << log_n), kThreads, 0, s, 
+    launch_chained(diagonal_mac_kernel<1>, grid_for((2LL * limbs) << log_n), kThreads, 0, s,
         t, log_n, limbs, prime_base, terms, x_stride, accumulate, y, y_stride);
   return cudaGetLastError();
 }
