@@ -6,7 +6,8 @@ the tile of the contiguous pass) on a batch of 24 limbs, forward and inverse, wi
 the engine's CUDA-event profiling; checks that the shape's words equal the default
 shape's (every shape performs the same butterflies); and writes the fastest shape
 per size to ``fhe_b200/ntt_tuning.json``, which the package installs when it loads
-the library.
+the library.  On these presets only the default shape runs the scaling primes in doubles,
+so it is the one to beat; another can win only on transforms that are all in integers.
 """
 from __future__ import annotations
 

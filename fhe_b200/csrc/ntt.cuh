@@ -645,12 +645,12 @@ __device__ __forceinline__ void ntt_pass_int(const NttPass &a, const PrimeTables
 // leave them; a CTA that loads any other word returns false before it stores anything, and
 // takes the integer pass.  Radix-16 rounds: against radix-8 at 256 threads that is one
 // exchange and one barrier instead of two at 8 stages, and twice the loads in flight
-// (hoisted rotations at N = 2^16: 1585 us with radix-8, 1501 with radix-16).
-// A loop over one round's body, to spare the instruction cache, measured slower (the index
-// arithmetic no longer folds): 558 against 429 us for the transforms below.
+// (hoisted rotations at N = 2^16, when it was chosen: 1585 us with radix-8, 1501 with
+// radix-16).  A loop over one round's body, to spare the instruction cache, measured slower
+// then (the index arithmetic no longer folds): 558 against 429 us for the transforms below.
 // Bound by latency and the FP64 pipe (40 % active).  Exact forward and inverse transform of
-// four ciphertexts of 24 limbs at N = 2^16: 694 us with every limb in integers, 429 us now
-// (2 x 201 MB in and out); one product at N = 2^17 and 76 levels: 6300 us, 4228 us.
+// four ciphertexts of 24 limbs at N = 2^16: 696 us with every limb in integers, 403 us now
+// (2 x 201 MB in and out).
 //
 // In a contiguous pass (of at most 9 stages) a warp owns 512 adjacent words, whole
 // sub-transforms, from load to store: its rounds exchange words inside the warp, and the
@@ -847,7 +847,11 @@ struct NttLimbOrder {
   uint8_t limb[kNttMaxLimbs] = {};
 };
 
-// Both kinds of limbs, a shape known at compile time.  80 registers and six CTAs an SM.
+// Both kinds of limbs, a shape known at compile time.  80 registers and six CTAs an SM; the
+// mixed passes, which hold the value, the exact and the integer form, spill for it (the lazy
+// rescale's by 100 to 160 bytes a thread, the tensor loader's, on the path without the fold,
+// by 260 and more).  Fewer loads in flight spill less and are slower: the tensor's transform of
+// a product at N = 2^17 608 us, 619 with four elements' loads at a time and 636 with two.
 template <int LOG_N, bool STRIDED, bool INVERSE, class Loader, class Storer, int VALUE_ONLY>
 __global__ void __launch_bounds__(kNttThreads, 6)
     ntt_pass_kernel(NttPass a, NttLimbOrder order, PrimeTables t, Loader load, Storer store) {
