@@ -248,7 +248,10 @@ extern "C" int fhe_relinearize_noalloc(fhe_engine *engine, const int64_t *ct_dev
     dp.inverse_r = scratch + int_words;
     dp.product_r = dp.inverse_r + static_cast<size_t>(dp.count) * 16;
     dp.product_r_squared = dp.product_r + static_cast<size_t>(dp.count) * 256;
-    const PrimeTables &t = e.tables();
+    // Without the tables that a caller's transform shape has made on first use, unless they
+    // are there: the exact butterflies give the same words.
+    PrimeTables t = e.tables();
+    if (t.shoup_tables->root == nullptr) t.shoup_tables = nullptr;
     note_launch();
     noalloc_partition_constants_kernel<<<dp.count, 256, 0, s>>>(lay, t.q, t.r_squared, dints,
                                                                 dp.inverse_r, dp.product_r,

@@ -92,6 +92,41 @@ def test_noalloc_relinearize_allocates_no_device_memory():
     e.close()
 
 
+def test_noalloc_allocates_nothing_under_a_callers_transform_shape():
+    """A shape in integers has tables of its own, made by the first transform that needs
+    them: not by this call."""
+    from fhe_b200 import Engine, RELINEARIZATION_KEY, _lib
+
+    lib = _lib.load()
+    e = Engine(log_coeff_count=14, special_prime_count=1)
+    mid = e.moduli_id(e.max_key_switching_level)
+    L = e.chains(mid)
+    rng = np.random.default_rng(101)
+    key = uniform_limbs(rng, e.moduli[mid:], 2 * e.partition_count(mid), e.coeff_count)
+    rk = e.upload(key, mid, NTT | SPECIAL, RELINEARIZATION_KEY)
+    ct = e.upload(uniform_limbs(rng, e.moduli[mid:mid + L], 3, e.coeff_count), mid, NTT)
+    out = e.upload(np.zeros((2, L, e.coeff_count), dtype=np.int64), mid)
+    want = e.relinearize(ct, rk).download()
+    saved = [ctypes.c_int() for _ in range(3)]
+    assert lib.fhe_ntt_tuning_get(14, *map(ctypes.byref, saved)) == 0
+    rc, msg = _noalloc(e, ct, mid, rk, mid, out)  # the first call resolves the array
+    assert rc == 0, msg
+    assert lib.fhe_ntt_tuning_set(14, 6, 2, 11) == 0
+    try:
+        before = _free_device_bytes()
+        rc, msg = _noalloc(e, ct, mid, rk, mid, out)
+        assert rc == 0, msg
+        assert _free_device_bytes() == before
+        assert np.array_equal(out.download(), want)
+        assert np.array_equal(e.relinearize(ct, rk).download(), want)  # makes the tables
+        rc, msg = _noalloc(e, ct, mid, rk, mid, out)
+        assert rc == 0, msg
+        assert np.array_equal(out.download(), want)
+    finally:
+        lib.fhe_ntt_tuning_set(14, *[v.value for v in saved])
+    e.close()
+
+
 def test_noalloc_rejects_sizes_beyond_its_scratch():
     from fhe_b200 import Engine, RELINEARIZATION_KEY
 
