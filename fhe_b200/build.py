@@ -23,17 +23,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
           "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include"), "-I", CSRC]
 
-# The transforms' files hold a kernel per ring size and fusion and compile in parts side by
-# side.  It changes the generated code: those kernels take the same time or up to 6 % less
-# (both transforms at N = 2^14: 12.0 us a call without it, 11.3 with it), the others more
-# (three partitions' key product at N = 2^16 57.8 us without, 71.1 with; the fused stage of a
-# bootstrap 3.70 and 4.22 ms, its level-downs 1.07 and 1.22 ms).
-SPLIT_COMPILED = ("ntt_forward.cu", "ntt_inverse.cu", "ntt_plain.cu", "ntt_rescale.cu",
-                  "ntt_tensor.cu", "ntt_value.cu")
-
-
-def arch_flags(src: str) -> list:
-    return ARCH + (["--split-compile=4"] if os.path.basename(src) in SPLIT_COMPILED else [])
+# Every source is compiled whole.  --split-compile, which compiles a file's kernels in parts side
+# by side, gives other code from one build to the next: the exact forward transforms of
+# ntt_forward.cu spilled 0 or 292 bytes, in turn, from the same source.
 
 
 def nvcc() -> str:
@@ -53,7 +45,7 @@ def _compile(src: str, verbose: bool, extra) -> str:
     newest = max([os.path.getmtime(src), os.path.getmtime(os.path.abspath(__file__))] + [os.path.getmtime(h) for h in _headers()])
     if os.path.exists(obj) and os.path.getmtime(obj) >= newest:
         return obj
-    cmd = [nvcc()] + arch_flags(src) + COMMON + list(extra) + ["-c", src, "-o", obj]
+    cmd = [nvcc()] + ARCH + COMMON + list(extra) + ["-c", src, "-o", obj]
     if src.endswith(".cpp"):
         cmd = [nvcc()] + COMMON + ["-Wno-deprecated-gpu-targets"] + list(extra) + ["-x", "c++", "-c", src, "-o", obj]
     if verbose:

@@ -847,13 +847,16 @@ struct NttLimbOrder {
   uint8_t limb[kNttMaxLimbs] = {};
 };
 
-// Both kinds of limbs, a shape known at compile time.  80 registers and six CTAs an SM; the
-// mixed passes, which hold the value, the exact and the integer form, spill for it (the lazy
-// rescale's by 100 to 160 bytes a thread, the tensor loader's, on the path without the fold,
-// by 260 and more).  Fewer loads in flight spill less and are slower: the tensor's transform of
-// a product at N = 2^17 608 us, 619 with four elements' loads at a time and 636 with two.
+// Both kinds of limbs, a shape known at compile time.  80 registers and six CTAs an SM where
+// values count (at five ModUp's transforms of a product at N = 2^17 take 1005 us, 977 at six);
+// the exact ones, which hold more constants, 96 and five (both transforms of a text at
+// N = 2^14 10.9 us a call, 11.9 at six; four inverse ones at N = 2^16 208 and 217).
+// The mixed passes, which hold the value, the exact and the integer form, spill at 80 (the lazy
+// rescale's by about 100 bytes a thread, the tensor loader's, on the path without the fold, by
+// 260 and more).  Fewer loads in flight spill less and are slower: the tensor's transform of
+// a product at N = 2^17 648 us, 652 with four elements' loads at a time and 688 with two.
 template <int LOG_N, bool STRIDED, bool INVERSE, class Loader, class Storer, int VALUE_ONLY>
-__global__ void __launch_bounds__(kNttThreads, 6)
+__global__ void __launch_bounds__(kNttThreads, VALUE_ONLY == kNttExact ? 5 : 6)
     ntt_pass_kernel(NttPass a, NttLimbOrder order, PrimeTables t, Loader load, Storer store) {
   chained_kernel_begin();
   __shared__ double tile[1 << kNttFpTileLog];

@@ -1,13 +1,20 @@
-"""Which sources the build compiles in parts (--split-compile changes the generated code)."""
-import glob
-import os
+"""The same sources give the same code: no flag whose result depends on how a build's work
+happens to be spread over threads."""
+import subprocess
 
 from fhe_b200 import build
 
 
-def test_only_the_transforms_are_compiled_in_parts():
-    sources = [os.path.basename(f) for f in glob.glob(os.path.join(build.CSRC, "*.cu"))]
-    assert {"bsgs.cu", "kernels.cu", "moddown_tc.cu", "modup_tc.cu", "rotate.cu"} < set(sources)
-    split = {f for f in sources if any("split-compile" in a for a in build.arch_flags(f))}
-    assert split == set(build.SPLIT_COMPILED)
-    assert all(f.startswith("ntt_") and f != "ntt_tc.cu" for f in split)
+def test_no_source_is_compiled_in_parts(monkeypatch, tmp_path):
+    commands = []
+    monkeypatch.setattr(build, "BUILD", str(tmp_path))
+    monkeypatch.setattr(build, "LIB", str(tmp_path / "lib.so"))
+
+    def run(cmd, check):
+        commands.append(cmd)
+        open(cmd[cmd.index("-o") + 1], "w").close()
+
+    monkeypatch.setattr(subprocess, "run", run)
+    build.build()
+    assert sum(c.endswith(".cu") for cmd in commands for c in cmd) >= 15
+    assert not [cmd for cmd in commands if any("split-compile" in a for a in cmd)]
